@@ -249,10 +249,7 @@ tb_status q8_gemm(const Q8Op& a, const Q8Op& b, std::vector<int4>& plan, int M, 
   c.beta = beta;
   c.tri = tri;
   c.flops = flops;
-  c.tiles = upload_tiles(plan, st);
-  if (!c.tiles) return TB_ERROR_ALLOC;
-  c.num_tiles = (int)plan.size();
-  return gemm_launch(c, st);
+  return gemm_launch_plan(c, plan, st);
 }
 
 char* q8_scratch(size_t bytes) {

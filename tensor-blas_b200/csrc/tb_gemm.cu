@@ -98,13 +98,13 @@ tb_status make_map8(CUtensorMap* map, const Operand& op, int box_rows) {
 }
 
 // Tensor map for the fp32 output C (rows x cols, column-major, ldc), box
-// {128 rows, 32 cols}, used by the TMA epilogue for loads and stores.
-bool make_c_map(CUtensorMap* map, float* C, long long rows, long long cols, long long ldc) {
+// {128 rows, box_cols}, used by the TMA epilogue for loads and stores.
+bool make_c_map(CUtensorMap* map, float* C, long long rows, long long cols, long long ldc, int box_cols) {
   EncodeTiledFn enc = encode_fn();
   if (!enc || (reinterpret_cast<uintptr_t>(C) & 15) != 0 || (ldc * 4) % 16 != 0) return false;
   cuuint64_t dims[2] = {(cuuint64_t)rows, (cuuint64_t)cols};
   cuuint64_t strides[1] = {(cuuint64_t)ldc * 4};
-  cuuint32_t box[2] = {128, 32};
+  cuuint32_t box[2] = {128, (cuuint32_t)box_cols};
   cuuint32_t estr[2] = {1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -113,13 +113,13 @@ bool make_c_map(CUtensorMap* map, float* C, long long rows, long long cols, long
 
 // Tensor map for an fp16 side copy restricted to rows x cols (the TMA store
 // clips to this extent, which implements the out_m / out_n region).
-bool make_half_out_map(CUtensorMap* map, __half* p, long long rows, long long cols, long long ld) {
+bool make_half_out_map(CUtensorMap* map, __half* p, long long rows, long long cols, long long ld, int box_cols) {
   EncodeTiledFn enc = encode_fn();
   if (!enc || !p || rows <= 0 || cols <= 0 || (reinterpret_cast<uintptr_t>(p) & 15) != 0 || (ld * 2) % 16 != 0)
     return false;
   cuuint64_t dims[2] = {(cuuint64_t)rows, (cuuint64_t)cols};
   cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2] = {128, 32};
+  cuuint32_t box[2] = {128, (cuuint32_t)box_cols};
   cuuint32_t estr[2] = {1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
              CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -177,7 +177,7 @@ tb_status launch_pair(const GemmArgs& args, int num_tiles, cudaStream_t stream, 
   const int pairs_max = sm_count() / 2;
   const int pairs = num_tiles < pairs_max ? num_tiles : pairs_max;
   void* tok = prof_begin(stream, kProfPair);
-  TB_CUDA_TRY(launch_engine(gemm_pair_kernel<Cfg>, 2 * pairs, Cfg::THREADS, Cfg::SMEM_BYTES, stream, args));
+  TB_CUDA_TRY(launch_engine(gemm_pair_kernel<Cfg>, 2 * pairs, kGemmThreads, Cfg::SMEM_BYTES, stream, args));
   prof_end(tok, stream, flops, bytes);
   note_launch();
   return TB_SUCCESS;
@@ -195,7 +195,7 @@ tb_status launch_variant(const GemmArgs& args, int num_tiles, cudaStream_t strea
   }
   int grid = num_tiles < sm_count() ? num_tiles : sm_count();
   void* tok = prof_begin(stream, kProfGemm);
-  TB_CUDA_TRY(launch_engine(gemm_kernel<Cfg, GROUPED>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, args));
+  TB_CUDA_TRY(launch_engine(gemm_kernel<Cfg, GROUPED>, grid, kGemmThreads, Cfg::SMEM_BYTES, stream, args));
   prof_end(tok, stream, flops, bytes);
   note_launch();
   return TB_SUCCESS;
@@ -215,16 +215,6 @@ int split_kchunk() {
     return (v >= 1 && v <= 64) ? v : 4;
   }();
   return k;
-}
-
-// CTA-pair epilogues load C one chunk ahead; TB_GEMM_C_AHEAD=0 in the
-// environment turns it off (read once).
-static bool c_ahead_enabled() {
-  static const int on = [] {
-    const char* e = getenv("TB_GEMM_C_AHEAD");
-    return (e && e[0] == '0') ? 0 : 1;
-  }();
-  return on == 1;
 }
 
 // CTA-pair launches that store from registers get a seventh operand stage
@@ -247,9 +237,8 @@ int gemm_bn(Split s, int kblocks) {
 
 tb_status gemm_build_args(const GemmCall& c, GemmArgs* out) {
   const bool split = c.split == Split::kHiLo && !c.fp8;
-  // pair launches: each CTA loads half of the tile's B rows (128 of 256;
-  // split: 64 of 128)
-  const int bn = c.fp8 ? kGemmBNFp8 : (c.pair ? (split ? 64 : 128) : gemm_bn(c.split, c.kblocks));
+  // pair launches: each CTA loads half of the tile's B rows (128 of 256)
+  const int bn = c.fp8 ? kGemmBNFp8 : (c.pair ? 128 : gemm_bn(c.split, c.kblocks));
   GemmArgs& a = *out;
   memset(&a, 0, sizeof(a));
   if (c.fp8) {
@@ -286,7 +275,7 @@ tb_status gemm_build_args(const GemmCall& c, GemmArgs* out) {
   a.diag = c.diag;
   a.corr_scale = c.corr_scale;
   a.kchunk = c.fp8 ? 1 : (c.kchunk > 0 ? c.kchunk : 1);
-  a.tma_c = make_c_map(&a.mapC, c.C, c.M, c.N, c.ldc) ? 1 : 0;
+  a.tma_c = make_c_map(&a.mapC, c.C, c.M, c.N, c.ldc, c.epi_cols) ? 1 : 0;
   a.out_hi = c.out_hi;
   a.out_lo = c.out_lo;
   a.ld_out = c.ld_out;
@@ -294,9 +283,9 @@ tb_status gemm_build_args(const GemmCall& c, GemmArgs* out) {
   a.out_m = c.out_m >= 0 ? (c.out_m < c.M ? c.out_m : c.M) : c.M;
   a.out_n = c.out_n >= 0 ? (c.out_n < c.N ? c.out_n : c.N) : c.N;
   a.tma_out = 0;
-  a.c_ahead = c_ahead_enabled() ? 1 : 0;
-  if (c.out_hi && a.tma_c && c.tri == 0 && make_half_out_map(&a.mapOut[0], c.out_hi, a.out_m, a.out_n, c.ld_out) &&
-      (!c.out_lo || make_half_out_map(&a.mapOut[1], c.out_lo, a.out_m, a.out_n, c.ld_out)))
+  if (c.out_hi && a.tma_c && c.tri == 0 &&
+      make_half_out_map(&a.mapOut[0], c.out_hi, a.out_m, a.out_n, c.ld_out, c.epi_cols) &&
+      (!c.out_lo || make_half_out_map(&a.mapOut[1], c.out_lo, a.out_m, a.out_n, c.ld_out, c.epi_cols)))
     a.tma_out = 1;
   a.err = c.err ? c.err : device_error_word();
   // TMA coordinates along the contiguous dimension must be 16-byte aligned.
@@ -323,64 +312,44 @@ static double gemm_algorithmic_bytes(const GemmCall& c) {
   return ops + cbytes + side;
 }
 
-tb_status gemm_launch(const GemmCall& c, cudaStream_t stream) {
+tb_status gemm_launch(GemmCall& c, cudaStream_t stream) {
   if (c.num_tiles <= 0) return TB_SUCCESS;
   GemmArgs a;
+  c.epi_cols = kEpiCols;
   TB_TRY(gemm_build_args(c, &a));
   const double bytes = gemm_algorithmic_bytes(c);
   const bool split = c.split == Split::kHiLo;
   const bool amn = c.a_hi.mn_major, bmn = c.b_hi.mn_major;
-  if (c.fp8) return launch_variant<GemmCfg<kGemmBNFp8, 1, false, false, false, true>, false>(a, c.num_tiles, stream,
-                                                                                            c.flops, bytes);
-  if (c.pair && split) {
-    if (amn && bmn) return launch_pair<PairCfg<true, true, false, 3>>(a, c.num_tiles, stream, c.flops, bytes);
-    if (amn && !bmn) return launch_pair<PairCfg<true, false, false, 3>>(a, c.num_tiles, stream, c.flops, bytes);
-    if (!amn && !bmn) return launch_pair<PairCfg<false, false, false, 3>>(a, c.num_tiles, stream, c.flops, bytes);
-    return launch_pair<PairCfg<false, true, false, 3>>(a, c.num_tiles, stream, c.flops, bytes);
+  // one instantiation per operand layout of a family of configurations
+#define TB_BY_LAYOUT(LAUNCH, ...)                                               \
+  do {                                                                          \
+    if (amn && bmn) return LAUNCH(true, true, ##__VA_ARGS__);                   \
+    if (amn && !bmn) return LAUNCH(true, false, ##__VA_ARGS__);                 \
+    if (!amn && !bmn) return LAUNCH(false, false, ##__VA_ARGS__);               \
+    return LAUNCH(false, true, ##__VA_ARGS__);                                  \
+  } while (0)
+#define TB_PAIR(AMN, BMN, MODE) launch_pair<PairCfg<AMN, BMN, MODE>>(a, c.num_tiles, stream, c.flops, bytes)
+#define TB_SINGLE(AMN, BMN, BN, NS, PF) \
+  launch_variant<GemmCfg<BN, NS, AMN, BMN, PF>, false>(a, c.num_tiles, stream, c.flops, bytes)
+  if (c.fp8) {
+    if (c.pair) return TB_PAIR(false, false, PairMode::kFp8);
+    return launch_variant<GemmCfg<kGemmBNFp8, 1, false, false, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
   }
+  if (c.pair && split) TB_BY_LAYOUT(TB_PAIR, PairMode::kSplit);
   if (c.pair) {
     const int direct = pair_direct_mode();
-    if (direct == 2 || (direct == 1 && c.beta == 0.f && !c.out_hi)) {
-      if (amn && bmn) return launch_pair<PairCfg<true, true, true>>(a, c.num_tiles, stream, c.flops, bytes);
-      if (amn && !bmn) return launch_pair<PairCfg<true, false, true>>(a, c.num_tiles, stream, c.flops, bytes);
-      if (!amn && !bmn) return launch_pair<PairCfg<false, false, true>>(a, c.num_tiles, stream, c.flops, bytes);
-      return launch_pair<PairCfg<false, true, true>>(a, c.num_tiles, stream, c.flops, bytes);
-    }
-    if (amn && bmn) return launch_pair<PairCfg<true, true>>(a, c.num_tiles, stream, c.flops, bytes);
-    if (amn && !bmn) return launch_pair<PairCfg<true, false>>(a, c.num_tiles, stream, c.flops, bytes);
-    if (!amn && !bmn) return launch_pair<PairCfg<false, false>>(a, c.num_tiles, stream, c.flops, bytes);
-    return launch_pair<PairCfg<false, true>>(a, c.num_tiles, stream, c.flops, bytes);
+    if (direct == 2 || (direct == 1 && c.beta == 0.f && !c.out_hi)) TB_BY_LAYOUT(TB_PAIR, PairMode::kDirect);
+    TB_BY_LAYOUT(TB_PAIR, PairMode::kStaged);
   }
-  if (c.kblocks > 0 && c.kblocks <= kGemmPfMaxKb) {
-    if (!split) {
-      if (amn && bmn) return launch_variant<GemmCfg<128, 1, true, true, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-      if (amn && !bmn) return launch_variant<GemmCfg<128, 1, true, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-      if (!amn && !bmn)
-        return launch_variant<GemmCfg<128, 1, false, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-      return launch_variant<GemmCfg<128, 1, false, true, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    }
-    if (amn && bmn) return launch_variant<GemmCfg<128, 3, true, true, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    if (amn && !bmn) return launch_variant<GemmCfg<128, 3, true, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    if (!amn && !bmn) return launch_variant<GemmCfg<128, 3, false, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    return launch_variant<GemmCfg<128, 3, false, true, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-  }
-  if (!split && engine_override() == kEngineNarrow) {  // plans built with gemm_bn() = 128
-    if (amn && bmn) return launch_variant<GemmCfg<128, 1, true, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    if (amn && !bmn) return launch_variant<GemmCfg<128, 1, true, false>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    if (!amn && !bmn) return launch_variant<GemmCfg<128, 1, false, false>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    return launch_variant<GemmCfg<128, 1, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-  }
-  if (!split) {
-    if (amn && bmn) return launch_variant<GemmCfg<256, 1, true, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    if (amn && !bmn) return launch_variant<GemmCfg<256, 1, true, false>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    if (!amn && !bmn) return launch_variant<GemmCfg<256, 1, false, false>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    return launch_variant<GemmCfg<256, 1, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-  } else {
-    if (amn && bmn) return launch_variant<GemmCfg<128, 3, true, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    if (amn && !bmn) return launch_variant<GemmCfg<128, 3, true, false>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    if (!amn && !bmn) return launch_variant<GemmCfg<128, 3, false, false>, false>(a, c.num_tiles, stream, c.flops, bytes);
-    return launch_variant<GemmCfg<128, 3, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
-  }
+  const bool pf = c.kblocks > 0 && c.kblocks <= kGemmPfMaxKb;
+  if (split && pf) TB_BY_LAYOUT(TB_SINGLE, 128, 3, true);
+  if (split) TB_BY_LAYOUT(TB_SINGLE, 128, 3, false);
+  if (pf) TB_BY_LAYOUT(TB_SINGLE, 128, 1, true);
+  if (gemm_bn(c.split, c.kblocks) == 128) TB_BY_LAYOUT(TB_SINGLE, 128, 1, false);
+  TB_BY_LAYOUT(TB_SINGLE, 256, 1, false);
+#undef TB_SINGLE
+#undef TB_PAIR
+#undef TB_BY_LAYOUT
 }
 
 // Large plain launches run on CTA pairs; TB_GEMM_PAIR=0 in the environment
@@ -390,15 +359,9 @@ static thread_local int t_engine_override = -1;
 void set_engine_override(int engine) { t_engine_override = engine; }
 int engine_override() { return t_engine_override; }
 
-// Long split launches (hi/lo operands, three products) that write no FP16
-// side copies run on CTA pairs too (256 x 128 tiles); TB_GEMM_PAIR_SPLIT=0
-// in the environment keeps them on single-CTA 128 x 128 tiles (read once).
-// On a B200: split SYRK n = k = 16384 11.62-11.67 ms on pairs against
-// 12.22-12.37 ms, results bit-identical; the split TRSM's long updates
-// (which stage the next leaf's hi/lo copies) took 1 % longer on pairs and
-// stay on single CTAs. Per SM a 256 x 128 pair MMA runs as long as the
-// single-CTA 128 x 128 one, so the pair saves shared-memory and L2 traffic
-// only; a 256-column split tile would need 256 fold registers per thread.
+// Long split launches (hi/lo operands, three products) run on CTA pairs too
+// (256 x 256 tiles); TB_GEMM_PAIR_SPLIT=0 in the environment keeps them on
+// single-CTA 128 x 128 tiles (read once).
 static bool pair_split_enabled() {
   static const bool on = [] {
     const char* e = getenv("TB_GEMM_PAIR_SPLIT");
@@ -470,35 +433,49 @@ static tb_status set_tiles(GemmCall& c, const std::vector<int4>& tiles, int work
   return TB_SUCCESS;
 }
 
-tb_status gemm_launch_plan(GemmCall& c, const std::vector<int4>& plan, cudaStream_t stream) {
-  const bool pf = c.kblocks > 0 && c.kblocks <= kGemmPfMaxKb;
-  c.pair = !c.fp8 && (c.split == Split::kPlain || (pair_split_enabled() && !c.out_hi)) && !pf && c.M >= 512 &&
-           c.N >= 512 && pair_engine_enabled();
-  if (!c.pair) {
-    TB_TRY(set_tiles(c, plan, std::min<int>((int)plan.size(), sm_count()), stream));
-    return gemm_launch(c, stream);
-  }
-  // merge vertically adjacent 128-row tiles into 256-row pair tiles (the K
-  // range of a pair tile spans both halves; products outside an operand's
-  // support multiply stored zeros, and masked outputs are never written)
-  // (a flat index over (256-row block, 128-column block): plans have
-  // thousands of tiles and this runs on every call)
+// Vertically and horizontally adjacent tiles of a plan merged into 256 x 256
+// pair tiles (the K range of a pair tile spans its parts; products outside an
+// operand's support multiply stored zeros, and masked outputs are never
+// written).
+static std::vector<int4> merge_pairs(const std::vector<int4>& plan, int M, int N) {
+  // a flat index over 256 x 256 blocks: plans have thousands of tiles and
+  // this runs on every call
   std::vector<int4> merged;
   merged.reserve(plan.size());
-  const long long rb = ((long long)c.M + 255) / 256, cb = ((long long)c.N + 127) / 128;
+  const long long rb = ((long long)M + 255) / 256, cb = ((long long)N + 255) / 256;
   std::vector<int> where((size_t)(rb * cb), -1);
   for (const int4& t : plan) {
-    int& w = where[(size_t)((long long)(t.x >> 8) * cb + (t.y >> 7))];
+    int& w = where[(size_t)((long long)(t.x >> 8) * cb + (t.y >> 8))];
     if (w < 0) {
       w = (int)merged.size();
-      merged.push_back(make_int4((t.x >> 8) << 8, t.y, t.z, t.w));
+      merged.push_back(make_int4((t.x >> 8) << 8, (t.y >> 8) << 8, t.z, t.w));
     } else {
       int4& m = merged[w];
       m.z = t.z < m.z ? t.z : m.z;
       m.w = t.w > m.w ? t.w : m.w;
     }
   }
-  TB_TRY(set_tiles(c, merged, std::min<int>((int)merged.size(), sm_count() / 2), stream));
+  return merged;
+}
+
+tb_status gemm_launch_plan(GemmCall& c, const std::vector<int4>& plan, cudaStream_t stream) {
+  const bool pf = c.kblocks > 0 && c.kblocks <= kGemmPfMaxKb;
+  c.pair = !pf && c.M >= 512 && c.N >= 512 && pair_engine_enabled() &&
+           (c.fp8 || c.split == Split::kPlain || pair_split_enabled());
+  std::vector<int4> merged;
+  if (c.pair) {
+    merged = merge_pairs(plan, c.M, c.N);
+    // split: a 256 x 256 pair tile takes about 1.45 times a 128 x 128 single
+    // CTA's time (four times the work at a better rate on two SMs), so the
+    // pairs lose where they leave more of the last wave empty
+    const long sms = sm_count(), ws = ((long)plan.size() + sms - 1) / sms,
+               wp = ((long)merged.size() + sms / 2 - 1) / (sms / 2);
+    if (!c.fp8 && c.split == Split::kHiLo && wp * 1.45 > (double)ws) c.pair = false;
+  }
+  if (c.pair)
+    TB_TRY(set_tiles(c, merged, std::min<int>((int)merged.size(), sm_count() / 2), stream));
+  else
+    TB_TRY(set_tiles(c, plan, std::min<int>((int)plan.size(), sm_count()), stream));
   return gemm_launch(c, stream);
 }
 

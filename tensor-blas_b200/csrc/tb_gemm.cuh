@@ -7,14 +7,15 @@
 // flattened recursion levels of SYRK/SYR2K (lower-triangle tile lists), the
 // off-diagonal updates and leaf products of TRSM, and TRMM/SYMM.
 //
-// Roles (192 threads, one CTA per SM):
-//   warp 0      TMA producer: 64-wide K slabs of A and B into a smem ring.
-//   warp 1      TMEM allocator + single-thread UMMA issuer.
-//   warps 2..5  epilogue: TMEM -> registers -> alpha/beta -> C.
-//   warp 6      (prefetch variants only, 224 threads) C loader: streams
-//               128 x 32 chunks of C into a ring of shared-memory slots.
-// The fp32 accumulator is double-buffered in TMEM (2 x 256 columns) so the
-// epilogue of tile t overlaps the MMAs of tile t+1.
+// Roles (384 threads, one CTA per SM):
+//   warp 0       TMA producer: 64-wide K slabs of A and B into a smem ring.
+//   warp 1       TMEM allocator + single-thread UMMA issuer.
+//   warp 2       C loader: streams 128 x 16 chunks of C into the epilogue's
+//                shared-memory slots ahead of their use.
+//   warps 4..11  epilogue, two groups of four warps, one half of the tile's
+//                columns each: TMEM -> registers -> alpha/beta -> C.
+// The fp32 accumulators are double-buffered in TMEM so the epilogue of tile t
+// overlaps the MMAs of tile t+1.
 //
 // Operands are fp16 in global memory, either MN-major (column-major storage
 // with the M/N index contiguous, the layout the reference's FP32->FP16
@@ -26,21 +27,24 @@
 //   K-major : TMA box {64 (K), R rows} -> R x 128 B; SBO = 1 KB between
 //             8-row groups; a K step of 16 advances the descriptor by 32 B.
 //
-// Output: each 128 x 32 chunk of the tile is staged in shared memory
+// Output: each 128 x 16 chunk of the tile is staged in shared memory
 // (column-major, 512 B per column) and written with one TMA tensor store, so
 // HBM sees 512-byte runs instead of one 128-byte piece per warp and column.
-// When beta != 0, or when a tile crosses the lower-triangle mask, the chunk
-// of C is first brought in with a TMA load and combined in shared memory
-// (masked elements keep their old value). A plain per-element path remains
-// for C that TMA cannot address (unaligned base or leading dimension).
+// When beta != 0 the chunk of C is first brought in with a TMA load and
+// combined in shared memory (masked elements keep their old value). A plain
+// per-element path serves C that TMA cannot address (unaligned base or
+// leading dimension) and masked tiles with beta = 0.
 //
 // Split ("3-product") mode holds hi and lo copies of both operands and runs
 //   acc0 += Ahi*Bhi ; acc1 += Ahi*Blo + Alo*Bhi
 // with the correction in its own TMEM accumulator (Ootomo & Yokota 2022,
 // the error-corrected FP16 scheme cuMpSGEMM's FP16TCEC mode uses). Every
-// `kchunk` K-blocks the epilogue folds acc0 + corr_scale * acc1 into FP32
-// registers with round-to-nearest adds: the tensor core's own FP32
-// accumulation truncates, which would cost ~K/16 ulps.
+// `kchunk` K-blocks the epilogue adds acc0 to FP32 registers with
+// round-to-nearest adds: the tensor core's own FP32 accumulation truncates,
+// which would cost ~K/16 ulps. The correction, 2^-11 of the result, stays in
+// its accumulator over the tile's whole K range and is added once: its
+// truncation is 2^-11 of the main accumulator's, and the fold reads half the
+// TMEM columns and rounds half as often.
 #pragma once
 #include "tb_ptx.cuh"
 
@@ -49,8 +53,8 @@ namespace tb {
 struct GemmArgs {
   CUtensorMap mapA[2];  // [0] hi, [1] lo (split mode only)
   CUtensorMap mapB[2];
-  CUtensorMap mapC;     // fp32 C, box {128, 32} (TMA epilogue only)
-  CUtensorMap mapOut[2];  // fp16 side copies hi / lo over [0,out_m) x [0,out_n), box {128, 32}
+  CUtensorMap mapC;     // fp32 C, box {128, 16} (TMA epilogue only)
+  CUtensorMap mapOut[2];  // fp16 side copies hi / lo over [0,out_m) x [0,out_n), box {128, 16}
   const int4* tiles;    // {m0, n0, kb_begin, kb_end}; m0/n0 relative to C
   int num_tiles;
   int a_off;  // row offset of the A operand in mapA's row coordinate
@@ -72,8 +76,7 @@ struct GemmArgs {
   long long ld_out;
   float out_lo_scale;
   int out_m, out_n;  // side copies only for rows < out_m and columns < out_n
-  int tma_out;       // 1: side copies through mapOut (requires tma_c and tri == 0)
-  int c_ahead;       // CTA-pair kernel: C chunks loaded one ahead where no side copies are staged
+  int tma_out;       // 1: side copies through mapOut where they are staged (requires tma_c and tri == 0)
   int* err;
   // FP8: per-(128-row block, 128-deep K block) scales of the A and B
   // operands, row-block-major with scale_ld K blocks per row block.
@@ -111,17 +114,18 @@ __device__ __forceinline__ int static_next(const GemmArgs& a, int b, int nb, int
 constexpr int kTileQ = 4;
 
 // The next tile of a consumer role: static striding, or the producer's
-// queue (q/ph: the role's ring position). EPI: called by all 128 epilogue
-// threads together, which then agree on the result.
+// queue (q/ph: the role's ring position). EPI: called by the 128 threads of
+// an epilogue group together, which then agree on the result (named barrier
+// `bar`).
 template <bool EPI>
 __device__ __forceinline__ int next_tile(const GemmArgs& args, int t, const volatile int* tq_idx, uint64_t* tq_full,
                                          uint64_t* tq_empty, int& q, uint32_t& ph, volatile int* abort_flag,
-                                         int code) {
+                                         int code, int bar = 1) {
   if (!args.sched) return t < 0 ? static_first(args, blockIdx.x) : static_next(args, blockIdx.x, gridDim.x, t);
   const bool got = mbar_wait(&tq_full[q], ph, abort_flag, args.err, code);
   int v = got ? tq_idx[q] : -1;
   if constexpr (EPI) {
-    if (named_bar_any(1, 128, !got)) v = -1;
+    if (named_bar_any(bar, 128, !got)) v = -1;
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(&tq_empty[q]);
   } else {
@@ -145,46 +149,65 @@ __device__ __forceinline__ const GemmArgs& tile_problem(const GemmArgs& args, in
   }
 }
 
-// PF (prefetch) variants serve launches whose tiles have few K-blocks: there
-// the epilogue, not the MMA, bounds the tile, so they trade pipeline stages
-// for a ring of shared-memory slots of 128 x 32 fp32 C chunks. A dedicated
-// loader warp fills the ring in the epilogue's chunk order, each slot as
-// soon as the stores of the chunk that used it last have read it, so the
-// next tile's C is in flight while this tile's epilogue runs (for chunks the
-// epilogue does not read, the loader only arrives on the slot's barrier).
-// fp16 side copies get two staging buffers.
+// Epilogue: two groups of four warps, each with one half of the tile's
+// columns, its own C slots and its own named barrier, in rolled loops over
+// chunks of 16 columns. What bounded the short launches was neither the MMAs
+// nor memory but instruction fetch: with four warps and the fold's 128
+// register sums handed to four unrolled 32-column copies of the store code, a
+// launch of four 128 x 128 tiles with 4 K-blocks took 22 us, of which the MMAs
+// were 2, and a TRSM leaf product of 512 x 16384 42.6 us. A group now runs one
+// short copy of the chunk code on 16 columns at a time, read back from TMEM
+// (split: the folded tile replaces its correction there) or picked out of the
+// fold's registers (pick16): 15 and 35 us. C (TMA slots) or the old values
+// (per-element path) are on their way before the accumulator is: a leaf
+// product of 6003 x 512 with an odd leading dimension went from 73 to 30 us,
+// the 512-instance batch from 6.5 to 5.1 ms.
+constexpr int kEpiGroups = 2;
+constexpr int kEpiCols = 16;
+constexpr int kEpiWarp0 = 4;  // first epilogue warp
+constexpr int kGemmThreads = 32 * (kEpiWarp0 + 4 * kEpiGroups);
+
+// Shared memory left beside the operand stages goes to the C slots: a group's
+// loader ring runs that many 8 KB chunks ahead of its epilogue.
+// PF variants serve launches whose tiles have few K-blocks: there the
+// epilogue, not the MMA, bounds the tile, so they trade operand stages for C
+// slots and for staging buffers of the fp16 side copies.
 // FP8 variant: e4m3 K-major operands scaled per 128 x 128 block; the
 // accumulator is folded into fp32 registers after every 128-deep K block
 // with the product of the two blocks' scales.
 template <int BN_, int NSPLIT_, bool A_MN_, bool B_MN_, bool PF_ = false, bool FP8_ = false>
 struct GemmCfg {
+  static constexpr bool PF = PF_;
   static constexpr bool FP8 = FP8_;
   static constexpr int ELEM = FP8 ? 1 : 2;       // operand bytes per element
   static constexpr int BM = 128, BN = BN_, BK = 128 / ELEM;  // one 128-byte swizzle row of K per stage
   static constexpr int KSTEPS = 4;               // MMAs per stage (K = 16 fp16 / 32 fp8 each)
   static constexpr int NSPLIT = NSPLIT_;
   static constexpr bool A_MN = A_MN_, B_MN = B_MN_;
-  static constexpr bool PF = PF_;
-  static constexpr bool FOLD = NSPLIT > 1 || FP8;  // accumulate in registers across TMEM rounds
-  static constexpr int NOPS = (NSPLIT == 1) ? 1 : 2;  // copies per operand (hi[, lo])
+  static constexpr bool SPLIT = NSPLIT > 1;
+  static constexpr bool FOLD = SPLIT || FP8;  // accumulate in registers across TMEM rounds
+  static constexpr int NOPS = SPLIT ? 2 : 1;  // copies per operand (hi[, lo])
   static constexpr int A_BYTES = BM * BK * ELEM;
   static constexpr int B_BYTES = BN * BK * ELEM;
   static constexpr int STAGE_BYTES = NOPS * (A_BYTES + B_BYTES);
-  static constexpr int STAGES = FP8 ? 6 : PF ? (NSPLIT == 1 ? 3 : 2) : ((STAGE_BYTES <= 48 * 1024) ? 4 : 3);
-  static constexpr int NACC = (NSPLIT == 1) ? 1 : 2;
-  static constexpr int ACC_COLS = NACC * BN;  // TMEM columns per accumulation buffer
-  static constexpr int TMEM_COLS = 2 * ACC_COLS;
+  static constexpr int STAGES = FP8 ? 6 : PF ? (SPLIT ? 2 : 3) : (SPLIT ? 3 : (BN == 128 ? 6 : 4));
+  // TMEM: two main accumulators (alternating by round), then two corrections
+  // (alternating by tile)
+  static constexpr int CORR_COL = 2 * BN;
+  static constexpr int TMEM_COLS = (SPLIT ? 4 : 2) * BN;
   static_assert(TMEM_COLS <= 512, "TMEM budget");
-  static constexpr int EPI_CHUNK_BYTES = 128 * 32 * 4;  // one staged 128 x 32 fp32 chunk
-  // C-chunk staging slots (and their load barriers); PF: the loader's ring
-  static constexpr int C_SLOTS = PF ? (NSPLIT == 1 ? 6 : 4) : 2;
-  static constexpr int SIDE_BYTES = PF ? 2 * EPI_CHUNK_BYTES : 0;  // PF: two fp16 hi/lo side buffers
-  static constexpr int EPI_BYTES = C_SLOTS * EPI_CHUNK_BYTES + SIDE_BYTES;
+  static constexpr int GC = BN / kEpiGroups;              // columns of one epilogue group
+  static constexpr int CHUNK_BYTES = 128 * kEpiCols * 4;  // one staged 128 x 16 fp32 chunk
+  static constexpr int C_SLOTS = PF ? (SPLIT ? 4 : 6) : 2;  // per group
+  static constexpr int SIDE = PF ? 2 : 0;                   // staging buffers for side copies, per group
+  static constexpr int GROUP_BYTES = (C_SLOTS + SIDE) * CHUNK_BYTES;
+  static constexpr int EPI_BYTES = kEpiGroups * GROUP_BYTES;
   static constexpr int BAR_BYTES = 512;
+  static_assert(8 * (2 * STAGES + 7 + 2 * kEpiGroups * C_SLOTS + 2 * kTileQ) + 4 * kTileQ + 8 <= BAR_BYTES,
+                "barrier space");
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + BAR_BYTES;
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
   static constexpr uint32_t IDESC = idesc_f16(BM, BN, false, A_MN, B_MN);
-  static constexpr int THREADS = PF ? 224 : 192;
 };
 
 template <bool MN, int ROWS>
@@ -213,55 +236,53 @@ __device__ __forceinline__ bool tile_reaches_mask(const GemmArgs& a, long long m
   return a.tri == 1 ? (m0 - (n0 + bn - 1)) < a.diag : (a.tri == 2 ? (n0 - (m0 + bm - 1)) < a.diag : false);
 }
 
-// Epilogue scalars, read into registers once per chunk. The epilogue's
+// Epilogue scalars, read into registers once per tile. The epilogue's
 // stores go through generic pointers (shared-memory slots, C, side copies)
-// that the compiler cannot tell apart from the kernel's parameter memory, so
-// GemmArgs fields read inside a store loop may be reloaded after every store.
+// that the compiler cannot tell apart from the kernel's parameter memory (or
+// a grouped launch's descriptor in global memory), so GemmArgs fields read
+// inside a store loop may be reloaded after every store.
 struct EpiK {
   float alpha, beta, lo_scale;
   int tri, diag;
   __device__ __forceinline__ explicit EpiK(const GemmArgs& a)
       : alpha(a.alpha), beta(a.beta), lo_scale(a.out_lo_scale), tri(a.tri), diag(a.diag) {}
-  // some element of the 128 x 32 chunk at (m0, n0) is masked
+  // some element of the 128 x W chunk at (m0, n0) is masked
+  template <int W>
   __device__ __forceinline__ bool chunk_masked(long long m0, long long n0) const {
-    return tri == 1 ? (m0 - (n0 + 31)) < diag : (tri == 2 ? (n0 - (m0 + 127)) < diag : false);
+    return tri == 1 ? (m0 - (n0 + W - 1)) < diag : (tri == 2 ? (n0 - (m0 + 127)) < diag : false);
   }
-  // The columns gj0 + [lo, hi) of row gi, out of the 32 from gj0 and below
+  // The columns gj0 + [lo, hi) of row gi, out of the W from gj0 and below
   // `ncols` (a bound on gj), that the mask keeps: one range per row, so the
   // element loops compare small ints instead of testing every element's
   // 64-bit (i, j) against the triangle (which cost more than the stores).
+  template <int W>
   __device__ __forceinline__ void keep_range(long long gi, long long gj0, long long ncols, int& lo, int& hi) const {
     long long h = ncols - gj0, l = 0;
     if (tri == 1) h = min(h, gi - diag + 1 - gj0);  // keep gj <= gi - diag
     if (tri == 2) l = gi + diag - gj0;              // keep gj >= gi + diag
-    hi = (int)max(0LL, min(32LL, h));
-    lo = (int)max(0LL, min(32LL, l));
+    hi = (int)max(0LL, min((long long)W, h));
+    lo = (int)max(0LL, min((long long)W, l));
   }
 };
 
-// New values of one row's 32 staged C elements: alpha v + beta old where
+// New values of one row's W staged C elements: alpha v + beta old where
 // unmasked (old kept where masked), written back in place.
-__device__ __forceinline__ void combine32(const EpiK& k, float* S, int row, const float* v, long long gi,
-                                          long long gj0, bool any_masked, float* r) {
-  if (any_masked) {
-    int lo, hi;
-    k.keep_range(gi, gj0, gj0 + 32, lo, hi);
+template <int W>
+__device__ __forceinline__ void combine(const EpiK& k, float* S, int row, const float* v, long long gi, long long gj0,
+                                        bool any_masked, float* r) {
+  int lo = 0, hi = W;
+  if (any_masked) k.keep_range<W>(gi, gj0, gj0 + W, lo, hi);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float old = S[j * 128 + row];
-      r[j] = (j >= lo && j < hi) ? fmaf(k.beta, old, k.alpha * v[j]) : old;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = fmaf(k.beta, S[j * 128 + row], k.alpha * v[j]);
+  for (int j = 0; j < W; ++j) {
+    const float old = S[j * 128 + row];
+    r[j] = (j >= lo && j < hi) ? fmaf(k.beta, old, k.alpha * v[j]) : old;
   }
 #pragma unroll
-  for (int j = 0; j < 32; ++j) S[j * 128 + row] = r[j];
+  for (int j = 0; j < W; ++j) S[j * 128 + row] = r[j];
 }
 
-// Scalars of the per-element store path for one tile, read into registers
-// once per tile (EpiK's fields plus C, bounds and the side-copy fields; in
-// grouped launches the problem descriptor lives in global memory).
+// Scalars of the per-element store path for one tile (EpiK's fields plus C,
+// bounds and the side-copy fields).
 struct StoreK : EpiK {
   float* C;
   long long ldc, ld_out;
@@ -273,15 +294,16 @@ struct StoreK : EpiK {
         out_lo(a.out_lo) {}
 };
 
-// Fused fp16 hi[/lo] copies of 32 result values of one row.
+// Fused fp16 hi[/lo] copies of W result values of one row.
+template <int W>
 __device__ __forceinline__ void store_fp16_copies(const StoreK& s, const float* r, long long gi, long long gj0) {
   const long long ld = s.ld_out;
   __half* hrow = s.out_hi + gi + gj0 * ld;
   __half* lrow = s.out_lo ? s.out_lo + gi + gj0 * ld : nullptr;
   int lo, hi;
-  s.keep_range(gi, gj0, s.out_n, lo, hi);
+  s.keep_range<W>(gi, gj0, s.out_n, lo, hi);
 #pragma unroll
-  for (int j = 0; j < 32; ++j) {
+  for (int j = 0; j < W; ++j) {
     if (j < lo || j >= hi) continue;
     const __half h = __float2half_rn(r[j]);
     hrow[(long long)j * ld] = h;
@@ -289,229 +311,380 @@ __device__ __forceinline__ void store_fp16_copies(const StoreK& s, const float* 
   }
 }
 
-// Per-element path: alpha/beta update of 32 consecutive columns of one row,
-// with the lower-triangle mask and bounds. With beta != 0 the 32 old values
-// are loaded before any store so the loads are in flight together.
-__device__ __forceinline__ void epilogue_store32(const StoreK& s, const float* v, long long gi, long long gj0) {
+// The old C values the per-element path needs for W consecutive columns of
+// one row (zeros where nothing is read), all loads in flight together.
+template <int W>
+__device__ __forceinline__ void load_old(const StoreK& s, float* old, bool row_ok, long long gi, long long gj0) {
+  int lo = 0, hi = 0;
+  if (row_ok) s.keep_range<W>(gi, gj0, s.N, lo, hi);
+  const float* crow = s.C + gi + gj0 * s.ldc;
+#pragma unroll
+  for (int j = 0; j < W; ++j) old[j] = (j >= lo && j < hi) ? __ldg(crow + (long long)j * s.ldc) : 0.f;
+}
+
+// Per-element path: alpha/beta update of W consecutive columns of one row,
+// with the triangle mask and bounds; old: load_old's values (read only when
+// beta != 0).
+template <int W>
+__device__ __forceinline__ void epilogue_store(const StoreK& s, const float* v, const float* old, long long gi,
+                                               long long gj0) {
   const long long ldc = s.ldc;
   float* crow = s.C + gi + gj0 * ldc;
   int lo, hi;
-  s.keep_range(gi, gj0, s.N, lo, hi);
-  bool keep[32];
+  s.keep_range<W>(gi, gj0, s.N, lo, hi);
+  float r[W];
+  const bool has_beta = s.beta != 0.0f;
 #pragma unroll
-  for (int j = 0; j < 32; ++j) keep[j] = j >= lo && j < hi;
-  float r[32];
-  if (s.beta != 0.0f) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = keep[j] ? __ldg(crow + (long long)j * ldc) : 0.f;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = fmaf(s.beta, r[j], s.alpha * v[j]);
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = s.alpha * v[j];
+  for (int j = 0; j < W; ++j) {
+    const float av = s.alpha * v[j];
+    r[j] = has_beta ? fmaf(s.beta, old[j], av) : av;
   }
 #pragma unroll
-  for (int j = 0; j < 32; ++j)
-    if (keep[j]) crow[(long long)j * ldc] = r[j];
-  if (s.out_hi && gi < s.out_m) store_fp16_copies(s, r, gi, gj0);
+  for (int j = 0; j < W; ++j)
+    if (j >= lo && j < hi) crow[(long long)j * ldc] = r[j];
+  if (s.out_hi && gi < s.out_m) store_fp16_copies<W>(s, r, gi, gj0);
 }
 
-// Epilogue state shared by the 4 epilogue warps (identical in all of them).
-struct EpiState {
-  int chunk;        // staged chunks written so far (selects the smem buffer)
-  uint32_t lphase;  // per-buffer phase bit of the C-load barriers
-  bool last_side;   // the previous chunk staged side copies (it used both buffers)
+// Side copies of one row's W values into a staged fp16 hi/lo chunk.
+template <int W>
+__device__ __forceinline__ void stage_side(const EpiK& k, __half* Hs, __half* Ls, const float* r, int row) {
+#pragma unroll
+  for (int j = 0; j < W; ++j) {
+    const __half hv = __float2half_rn(r[j]);
+    Hs[j * 128 + row] = hv;
+    Ls[j * 128 + row] = __float2half_rn((r[j] - __half2float(hv)) * k.lo_scale);
+  }
+}
+
+// Columns [16 c, 16 c + 16) of a thread's register sums: registers cannot be
+// indexed at run time, so one predicated copy per chunk position keeps a
+// single copy of the chunk code instead of one per chunk.
+template <int N>
+__device__ __forceinline__ void pick16(const float (&acc)[N], int c, float* v) {
+#pragma unroll
+  for (int q = 0; q < N / 16; ++q)
+    if (c == q) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = acc[16 * q + j];
+    }
+}
+
+// Whether a tile's chunks go through the C slots (TMA); the others are
+// stored per element. Masked tiles with beta == 0 store their unmasked
+// elements directly: the slots would first have to load C to keep the masked
+// ones.
+__device__ __forceinline__ bool tile_staged(const GemmArgs& P, bool masked) {
+  return P.tma_c && !(masked && P.beta == 0.0f);
+}
+
+// The C loader's walk (one thread): the CTA's tiles in the epilogue's chunk
+// order, the groups in turn; a group's chunk n goes to slot n % SLOTS of its
+// ring once the epilogue has given back the slot's previous chunk
+// (n - SLOTS). Chunks the epilogue does not read (beta == 0) only pass the
+// slot's barrier.
+template <int SLOTS, int STRIDE>
+struct CLoader {
+  float* stage;  // group g's slots start at stage + g * STRIDE
+  uint64_t *cfull, *cfree;
+  int slot[kEpiGroups];
+  uint32_t ph[kEpiGroups];
+  uint32_t armed, armed_phase;  // per slot: a load was armed / its phase
+
+  __device__ __forceinline__ CLoader(float* stage_, uint64_t* cfull_, uint64_t* cfree_)
+      : stage(stage_), cfull(cfull_), cfree(cfree_), armed(0), armed_phase(0) {
+    for (int g = 0; g < kEpiGroups; ++g) slot[g] = 0, ph[g] = 0;
+  }
+  // chunks of the tile at (m0, n0) with GC columns per group; false when a wait gave up
+  __device__ __forceinline__ bool tile(const GemmArgs& P, int m0, int n0, int gc, volatile int* abort_flag) {
+    const bool need = P.beta != 0.0f;
+    for (int c0 = 0; c0 < gc; c0 += kEpiCols) {
+#pragma unroll
+      for (int g = 0; g < kEpiGroups; ++g) {
+        const int gj = n0 + g * gc + c0;
+        if (gj >= P.N) continue;
+        const int s = g * SLOTS + slot[g];
+        if (!mbar_wait(&cfree[s], ph[g] ^ 1u, abort_flag, P.err, kDevErrTimeoutProducer)) return false;
+        if (need) {
+          mbar_arrive_expect_tx(&cfull[s], 128 * kEpiCols * 4);
+          tma_load_2d(stage + g * STRIDE + slot[g] * (128 * kEpiCols), &P.mapC, &cfull[s], m0, gj);
+          armed |= 1u << s;
+          armed_phase = (armed_phase & ~(1u << s)) | (ph[g] << s);
+        } else {
+          // the slot's earlier load was consumed before the slot came back
+          armed &= ~(1u << s);
+          mbar_arrive(&cfull[s]);
+        }
+        if (++slot[g] == SLOTS) {
+          slot[g] = 0;
+          ph[g] ^= 1u;
+        }
+      }
+    }
+    return true;
+  }
+  // every armed load lands before the CTA exits (immediate unless the
+  // epilogue left early)
+  __device__ __forceinline__ void drain(int* err) {
+    for (int i = 0; i < kEpiGroups * SLOTS; ++i) {
+      if (!((armed >> i) & 1u)) continue;
+      const uint64_t t0 = globaltimer_ns();
+      while (!mbar_try_wait(&cfull[i], (armed_phase >> i) & 1u))
+        if (globaltimer_ns() - t0 > 1000000000ull) {
+          if (err) atomicCAS(err, 0, kDevErrTimeoutTeardown);
+          break;
+        }
+    }
+  }
 };
 
-// TMA path for one 128 x 32 chunk at (m0, gj0): v[] holds this thread's row
-// (32 consecutive columns). All 128 epilogue threads call it together.
-// With TMA side copies (tma_out) the second staging buffer holds the fp16
-// hi/lo chunk (8 KB each) and the fp32 chunk is single-buffered; otherwise
-// chunks alternate between the two buffers. Problems of a grouped launch may
-// differ in this, so the wait before reusing a buffer looks at the previous
-// chunk's mode.
-__device__ __forceinline__ void epilogue_chunk_tma(const GemmArgs& args, float* stage, uint64_t* cload, EpiState& es,
-                                                   const float* v, int m0, int gj0, int row, bool need_load,
-                                                   bool issuer, volatile int* abort_flag) {
-  const EpiK k(args);
-  const bool side_mode = args.tma_out != 0;
-  const bool side = args.tma_out != 0 && gj0 < args.out_n && m0 < args.out_m;
-  const bool copies = !side_mode && args.out_hi && (long long)m0 + row < args.out_m;
-  const int b = side_mode ? 0 : (es.chunk & 1);
-  float* S = stage + b * (128 * 32);
-  __half* Hs = reinterpret_cast<__half*>(stage + 128 * 32);
-  __half* Ls = Hs + 128 * 32;
-  if (issuer) {
-    if (side_mode || es.last_side)
-      bulk_wait_read<0>();  // this chunk or the previous one uses both buffers: every earlier store has read smem
-    else
-      bulk_wait_read<1>();  // the store that last used buffer b has finished reading it
-    if (need_load) {
-      mbar_arrive_expect_tx(&cload[b], 128 * 32 * 4);
-      tma_load_2d(S, &args.mapC, &cload[b], m0, gj0);
-    }
-  }
-  named_bar_sync(1, 128);
-  const long long gi = (long long)m0 + row;
-  float r[32];
-  if (need_load) {
-    mbar_wait(&cload[b], (es.lphase >> b) & 1u, abort_flag, args.err, kDevErrTimeoutEpilogue);
-    es.lphase ^= 1u << b;
-    combine32(k, S, row, v, gi, gj0, k.chunk_masked(m0, gj0), r);
-  } else {
+// One epilogue group of four warps (128 threads, named barrier `bar`).
+template <int SLOTS, int SIDE>
+struct EpiGroup {
+  float* slots;               // the group's ring of 128 x 16 chunks, then SIDE fp16 hi/lo chunks
+  uint64_t *cfull, *cfree;    // per slot: chunk (or its hand-over) arrived / slot given back
+  int bar, row;               // row: this thread's row of the tile
+  bool issuer;
+  int slot = 0;        // next ring slot
+  uint32_t phase = 0;  // its barrier's phase (flips when the ring wraps)
+  int prev = -1;       // slot of the previous chunk, still to be released (-1: none)
+  int nside = 0;       // side-copy chunks staged so far (selects the buffer)
+
+  // One 128 x 16 chunk at (m0, gj) staged in the next slot: the slot holds
+  // this chunk of C when beta != 0; the result is combined in place and
+  // stored from the slot. Before the issuer stores a chunk it waits until the
+  // previous chunk's store has read its slot and gives that slot back to the
+  // loader. All 128 threads call it together; false, in every thread alike,
+  // when the slot's wait gave up. The FP16 side copies alternate between
+  // SIDE staging buffers, or (SIDE == 0) are stored from registers.
+  __device__ __forceinline__ bool chunk_staged(const GemmArgs& P, const StoreK& k, const float* v, int m0, int gj,
+                                               volatile int* abort_flag) {
+    constexpr int W = kEpiCols;
+    float* S = slots + slot * (128 * W);
+    const bool got = mbar_wait(&cfull[slot], phase, abort_flag, P.err, kDevErrTimeoutEpilogue);
+    const long long gi = (long long)m0 + row;
+    float r[W];
+    if (k.beta != 0.0f) {
+      combine<W>(k, S, row, v, gi, gj, k.chunk_masked<W>(m0, gj), r);
+    } else {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      r[j] = k.alpha * v[j];
-      S[j * 128 + row] = r[j];
+      for (int j = 0; j < W; ++j) {
+        r[j] = k.alpha * v[j];
+        S[j * 128 + row] = r[j];
+      }
     }
-  }
-  if (side) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const __half hv = __float2half_rn(r[j]);
-      Hs[j * 128 + row] = hv;
-      Ls[j * 128 + row] = __float2half_rn((r[j] - __half2float(hv)) * k.lo_scale);
+    const bool side = SIDE > 0 && P.tma_out && gj < k.out_n && m0 < k.out_m;
+    __half* Hs = reinterpret_cast<__half*>(slots + (SLOTS + (SIDE == 2 ? (nside & 1) : 0)) * (128 * W));
+    if constexpr (SIDE > 0) {
+      if (side) {
+        // two buffers: the store that used this one was read before the
+        // previous chunk's store was issued, which this thread has seen at the
+        // previous chunk's barrier
+        stage_side<W>(k, Hs, Hs + 128 * W, r, row);
+        ++nside;
+      }
     }
-  }
-  fence_proxy_async_smem();
-  named_bar_sync(1, 128);
-  if (issuer) {
-    tma_store_2d(&args.mapC, S, m0, gj0);
-    if (side) {
-      tma_store_2d(&args.mapOut[0], Hs, m0, gj0);
-      if (args.out_lo) tma_store_2d(&args.mapOut[1], Ls, m0, gj0);
+    fence_proxy_async_smem();
+    if (named_bar_any(bar, 128, !got)) return false;
+    if (issuer) {
+      bulk_wait_read<0>();  // the previous chunk's stores have read their slot and side buffer
+      if (prev >= 0) mbar_arrive(&cfree[prev]);
+      tma_store_2d(&P.mapC, S, m0, gj);
+      if (side) {
+        tma_store_2d(&P.mapOut[0], Hs, m0, gj);
+        if (k.out_lo) tma_store_2d(&P.mapOut[1], Hs + 128 * W, m0, gj);
+      }
+      bulk_commit();
     }
-    bulk_commit();
+    prev = slot;
+    if (++slot == SLOTS) {
+      slot = 0;
+      phase ^= 1u;
+    }
+    if (k.out_hi && !(SIDE > 0 && P.tma_out) && gi < k.out_m) store_fp16_copies<W>(k, r, gi, gj);
+    return true;
   }
-  if (copies) store_fp16_copies(StoreK(args), r, gi, gj0);
-  ++es.chunk;
-  es.last_side = side_mode;
-}
-
-// Pipelined form of the TMA path for tiles that load C and stage no side
-// copies: the C chunk for chunk c + 1 is requested (into the other buffer)
-// before chunk c is combined, so a tile pays one load latency instead of one
-// per chunk. c_issue_load requests chunk (m0, gj0) into buffer es.chunk + ahead
-// once every earlier store has read its buffer; epilogue_chunk_loaded then
-// combines and stores the chunk whose load was requested. Same arithmetic as
-// epilogue_chunk_tma.
-__device__ __forceinline__ void c_issue_load(const GemmArgs& args, float* stage, uint64_t* cload,
-                                             const EpiState& es, int ahead, int m0, int gj0) {
-  const int b = (es.chunk + ahead) & 1;
-  bulk_wait_read<0>();  // the store that last used buffer b (and every earlier one) has read it
-  mbar_arrive_expect_tx(&cload[b], 128 * 32 * 4);
-  tma_load_2d(stage + b * (128 * 32), &args.mapC, &cload[b], m0, gj0);
-}
-
-__device__ __forceinline__ void epilogue_chunk_loaded(const GemmArgs& args, float* stage, uint64_t* cload,
-                                                      EpiState& es, const float* v, int m0, int gj0, int row,
-                                                      bool issuer, volatile int* abort_flag) {
-  const EpiK k(args);
-  const int b = es.chunk & 1;
-  float* S = stage + b * (128 * 32);
-  const long long gi = (long long)m0 + row;
-  float r[32];
-  mbar_wait(&cload[b], (es.lphase >> b) & 1u, abort_flag, args.err, kDevErrTimeoutEpilogue);
-  es.lphase ^= 1u << b;
-  combine32(k, S, row, v, gi, gj0, k.chunk_masked(m0, gj0), r);
-  fence_proxy_async_smem();
-  named_bar_sync(1, 128);
-  if (issuer) {
-    tma_store_2d(&args.mapC, S, m0, gj0);
-    bulk_commit();
-  }
-  if (!args.tma_out && args.out_hi && gi < args.out_m) store_fp16_copies(StoreK(args), r, gi, gj0);
-  ++es.chunk;
-  es.last_side = false;
-}
-
-// PF epilogue, one 128 x 32 chunk (columns gj0..gj0+31) staged in the next
-// slot of the loader's ring. The slot holds this chunk of C when need_load
-// (the loader's TMA load completes its barrier) and is only handed over
-// otherwise; the result is combined in place and stored from the slot. Before
-// the issuer stores a chunk it waits until the previous chunk's stores have
-// read their slot and gives that slot back to the loader. Side copies
-// alternate between two fp16 buffers. All 128 epilogue threads call it
-// together and keep identical state. Returns false, in every thread alike,
-// when the slot's wait gave up.
-struct PfState {
-  int slot;        // next ring slot
-  uint32_t phase;  // its barrier's phase (flips when the ring wraps)
-  int prev;        // slot of the previous chunk, still to be released (-1: none)
-  int side;        // side-copy chunks written so far (selects the buffer)
 };
 
-template <int RING>
-__device__ __forceinline__ bool epilogue_chunk_pf(const GemmArgs& args, float* slots, __half* side_base,
-                                                  uint64_t* cfull, uint64_t* cfree, PfState& pf, const float* v,
-                                                  int m0, int gj0, int row, bool need_load, bool issuer,
-                                                  volatile int* abort_flag) {
-  const EpiK k(args);
-  const bool side = args.tma_out != 0 && gj0 < args.out_n && m0 < args.out_m;
-  const bool copies = !args.tma_out && args.out_hi && (long long)m0 + row < args.out_m;
-  const int slot = pf.slot;
-  float* S = slots + slot * (128 * 32);
-  __half* Hs = side_base + (pf.side & 1) * (2 * 128 * 32);
-  __half* Ls = Hs + 128 * 32;
-  const bool got = mbar_wait(&cfull[slot], pf.phase, abort_flag, args.err, kDevErrTimeoutEpilogue);
-  // also orders this chunk's smem writes after the issuer's previous stores
-  if (named_bar_any(1, 128, !got)) return false;
-  if (++pf.slot == RING) {
-    pf.slot = 0;
-    pf.phase ^= 1u;
-  }
-  const long long gi = (long long)m0 + row;
-  float r[32];
-  if (need_load) {
-    combine32(k, S, row, v, gi, gj0, k.chunk_masked(m0, gj0), r);
-  } else {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      r[j] = k.alpha * v[j];
-      S[j * 128 + row] = r[j];
+// The per-tile part of the epilogue. acc.begin() makes the group's
+// accumulators ready (waits for the MMAs, folds) and returns false when a
+// wait gave up; acc.chunk(c, v) gives columns [16 c, 16 c + 16) of the
+// group's GC. (m0, gy): the group's first row and column of C. False when
+// the epilogue has to stop.
+template <int GC, class Group, class Acc>
+__device__ __forceinline__ bool epilogue_tile(const GemmArgs& P, Group& g, Acc& acc, int m0, int gy, bool staged,
+                                              volatile int* abort_flag) {
+  const StoreK sk(P);
+  const long long gi = (long long)m0 + g.row;
+  const bool row_ok = gi < P.M;
+  const int nval = min(max((sk.N - gy + kEpiCols - 1) / kEpiCols, 0), GC / kEpiCols);  // chunks inside C
+  // per-element path: C's old values are loaded one chunk ahead, the first
+  // before the accumulator wait (where the fold leaves registers for it)
+  float old[kEpiCols];
+  const bool read_old = !staged && sk.beta != 0.0f;
+  if (Acc::kEarlyLoad && read_old) load_old<kEpiCols>(sk, old, row_ok, gi, gy);
+  if (named_bar_any(g.bar, 128, !acc.begin())) return false;
+  if (!Acc::kEarlyLoad && read_old) load_old<kEpiCols>(sk, old, row_ok, gi, gy);
+#pragma unroll 1
+  for (int c = 0; c < GC / kEpiCols; ++c) {
+    float v[kEpiCols];
+    acc.chunk(c, v);
+    if (c >= nval) continue;
+    const int gj = gy + c * kEpiCols;
+    if (staged) {
+      if (!g.chunk_staged(P, sk, v, m0, gj, abort_flag)) return false;
+    } else {
+      if (row_ok) epilogue_store<kEpiCols>(sk, v, old, gi, gj);
+      if (read_old && c + 1 < nval) load_old<kEpiCols>(sk, old, row_ok, gi, gj + kEpiCols);
     }
   }
-  if (side) {
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const __half hv = __float2half_rn(r[j]);
-      Hs[j * 128 + row] = hv;
-      Ls[j * 128 + row] = __float2half_rn((r[j] - __half2float(hv)) * k.lo_scale);
-    }
-  }
-  fence_proxy_async_smem();
-  named_bar_sync(1, 128);
-  if (issuer) {
-    // the previous chunk's stores have read their slot (and side buffer)
-    bulk_wait_read<0>();
-    if (pf.prev >= 0) mbar_arrive(&cfree[pf.prev]);
-    tma_store_2d(&args.mapC, S, m0, gj0);
-    if (side) {
-      tma_store_2d(&args.mapOut[0], Hs, m0, gj0);
-      if (args.out_lo) tma_store_2d(&args.mapOut[1], Ls, m0, gj0);
-    }
-    bulk_commit();
-  }
-  pf.prev = slot;
-  if (copies) store_fp16_copies(StoreK(args), r, gi, gj0);
-  if (side) ++pf.side;
   return true;
 }
 
+// FP8: the block scales of a tile's rounds, one round ahead of their use (a
+// load per round in the fold's path cost more than the round's MMAs).
+struct Fp8Scales {
+  const float *pa, *pb;
+  float na = 0.f, nb = 0.f;
+  // the scale rows of the 128-row block of A at C row m0 and of B at C column
+  // n0; blocks wholly outside C take the last one (their products are not stored)
+  __device__ __forceinline__ Fp8Scales(const GemmArgs& P, int m0, int n0, int kb0, int kb1) {
+    const int ra = (P.a_off + min(m0, P.M - 1)) >> 7, rb = (P.b_off + min(n0, P.N - 1)) >> 7;
+    pa = P.scale_a + (long long)ra * P.scale_ld + (P.k_off >> 7);
+    pb = P.scale_b + (long long)rb * P.scale_ld + (P.k_off >> 7);
+    if (kb0 < kb1) {
+      na = __ldg(pa + kb0);
+      nb = __ldg(pb + kb0);
+    }
+  }
+  __device__ __forceinline__ float next(int kb, int kb1) {
+    const float s = na * nb;
+    if (kb + 1 < kb1) {
+      na = __ldg(pa + kb + 1);
+      nb = __ldg(pb + kb + 1);
+    }
+    return s;
+  }
+};
+
+// Accumulators of one tile in the single-CTA kernel, as an epilogue group's
+// warp sees them (tmem: base + lane quarter + the group's first column).
+template <class Cfg>
+struct TileAcc {
+  static constexpr bool kEarlyLoad = true;
+  const GemmArgs& args;
+  const GemmArgs& P;
+  int4 tile;
+  int gc0;
+  uint32_t tmem;
+  uint64_t *tfull, *tempty, *xempty;
+  int &it, &nt;
+  volatile int* abort_flag;
+  float acc[Cfg::FOLD ? Cfg::GC : 16];
+  int buf = 0;
+  uint32_t folded = 0;  // split: TMEM columns of the folded tile
+
+  __device__ __forceinline__ void release(uint64_t* bar) {
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+  }
+  __device__ __forceinline__ bool round() {
+    buf = it & 1;
+    const uint32_t ph = (uint32_t)(it >> 1) & 1u;
+    ++it;
+    const bool got = mbar_wait(&tfull[buf], ph, abort_flag, args.err, kDevErrTimeoutEpilogue);
+    tc_fence_after();
+    return __all_sync(0xffffffffu, got);  // one decision per warp: TMEM loads follow
+  }
+  __device__ __forceinline__ bool begin() {
+    if constexpr (!Cfg::FOLD) {
+      return round();
+    } else {
+#pragma unroll
+      for (int j = 0; j < Cfg::GC; ++j) acc[j] = 0.f;
+      if constexpr (Cfg::FP8) {
+        Fp8Scales sc(P, tile.x, tile.y + gc0, tile.z, tile.w);
+        for (int kb = tile.z; kb < tile.w; ++kb) {  // kchunk = 1
+          const float s = sc.next(kb, tile.w);
+          if (!round()) return false;
+          const uint32_t ta = tmem + (uint32_t)(buf * Cfg::BN);
+#pragma unroll
+          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
+            float v[32];
+            tmem_ld32(ta + c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(s, v[j], acc[c0 + j]);
+          }
+          release(&tempty[buf]);
+        }
+      } else {
+        for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk) {
+          if (!round()) return false;
+          const uint32_t ta = tmem + (uint32_t)(buf * Cfg::BN);
+#pragma unroll
+          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
+            float v[32];
+            tmem_ld32(ta + c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
+          }
+          release(&tempty[buf]);
+        }
+        if (tile.z < tile.w) {  // the last round's commit covers the correction's MMAs
+          const uint32_t tc = tmem + (uint32_t)(Cfg::CORR_COL + (nt & 1) * Cfg::BN);
+#pragma unroll
+          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
+            float w[32];
+            tmem_ld32(tc + c0, w);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) w[j] = fmaf(args.corr_scale, w[j], acc[c0 + j]);
+            // the folded tile takes the place of the correction it was folded with
+            tmem_st32(tc + c0, w);
+          }
+          tmem_st_wait();
+          folded = tc;
+        }
+      }
+      return true;
+    }
+  }
+  __device__ __forceinline__ void chunk(int c, float* v) {
+    if constexpr (Cfg::FP8) {
+      pick16(acc, c, v);
+    } else if constexpr (Cfg::SPLIT) {
+      if (tile.z < tile.w) {
+        tmem_ld16(folded + (uint32_t)(c * kEpiCols), v);
+        if (c == Cfg::GC / kEpiCols - 1) {
+          release(&xempty[nt & 1]);
+          ++nt;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < kEpiCols; ++j) v[j] = 0.f;
+      }
+    } else {
+      tmem_ld16(tmem + (uint32_t)(buf * Cfg::BN + c * kEpiCols), v);
+      if (c == Cfg::GC / kEpiCols - 1) release(&tempty[buf]);  // fully read: hand it back to the MMA warp
+    }
+  }
+};
+
 template <class Cfg, bool GROUPED>
-__global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_constant__ GemmArgs args) {
+__global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_constant__ GemmArgs args) {
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES;
+  constexpr int kSlots = kEpiGroups * Cfg::C_SLOTS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* stage_c = reinterpret_cast<float*>(smem + STAGES * Cfg::STAGE_BYTES);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::STAGE_BYTES + Cfg::EPI_BYTES);
   uint64_t* empty = full + STAGES;
-  uint64_t* tfull = empty + STAGES;  // [2]
-  uint64_t* tempty = tfull + 2;      // [2]
-  uint64_t* drain = tempty + 2;      // [1] teardown barrier for the MMA issuer
-  uint64_t* cload = drain + 1;       // [C_SLOTS] C-chunk loads of the TMA epilogue
-  uint64_t* cfree = cload + Cfg::C_SLOTS;  // [C_SLOTS] PF: ring slots the epilogue gave back
-  uint64_t* tq_full = cfree + Cfg::C_SLOTS;  // [kTileQ] tile hand-off (device-side scheduler)
+  uint64_t* tfull = empty + STAGES;    // [2] main accumulator rounds
+  uint64_t* tempty = tfull + 2;        // [2]
+  uint64_t* xempty = tempty + 2;       // [2] correction accumulators given back
+  uint64_t* drain = xempty + 2;        // [1] teardown barrier for the MMA issuer
+  uint64_t* cfull = drain + 1;         // [group][C_SLOTS] C chunks of the loader's ring
+  uint64_t* cfree = cfull + kSlots;    // [group][C_SLOTS] ring slots the epilogue gave back
+  uint64_t* tq_full = cfree + kSlots;  // [kTileQ] tile hand-off (device-side scheduler)
   uint64_t* tq_empty = tq_full + kTileQ;     // [kTileQ]
   int* tq_idx = reinterpret_cast<int*>(tq_empty + kTileQ);  // [kTileQ]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tq_idx + kTileQ);
@@ -527,15 +700,16 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 4);
+      mbar_init(&tempty[b], 4 * kEpiGroups);
+      mbar_init(&xempty[b], 4 * kEpiGroups);
     }
-    for (int b = 0; b < Cfg::C_SLOTS; ++b) {
-      mbar_init(&cload[b], 1);
+    for (int b = 0; b < kSlots; ++b) {
+      mbar_init(&cfull[b], 1);
       mbar_init(&cfree[b], 1);
     }
     for (int b = 0; b < kTileQ; ++b) {
       mbar_init(&tq_full[b], 1);
-      mbar_init(&tq_empty[b], 1 + 4 + (Cfg::PF ? 1 : 0));  // MMA issuer, epilogue warps, C loader
+      mbar_init(&tq_empty[b], 2 + 4 * kEpiGroups);  // MMA issuer, C loader, epilogue warps
     }
     mbar_init(drain, 1);
     *abort_flag = 0;
@@ -549,10 +723,6 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
       tma_prefetch_map(&args.mapB[1]);
     }
     if (args.tma_c) tma_prefetch_map(&args.mapC);
-    if (args.tma_out) {
-      tma_prefetch_map(&args.mapOut[0]);
-      if (args.out_lo) tma_prefetch_map(&args.mapOut[1]);
-    }
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
@@ -639,12 +809,15 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    // Accumulation "chunks": plain mode accumulates a tile's whole K range in
-    // one TMEM buffer; split mode closes a chunk every `kchunk` K-blocks.
+    // Main accumulation in rounds, one TMEM buffer each: plain mode runs a
+    // tile's whole K range in one round; split mode closes a round every
+    // `kchunk` K-blocks and FP8 every K-block. Split mode's correction
+    // products go to the tile's own accumulator over all its rounds.
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 0;
-      int it = 0;  // chunk counter (selects TMEM buffer and phase)
+      int it = 0;  // round counter (selects the main buffer and its phase)
+      int nt = 0;  // tile counter (selects the correction buffer and its phase)
       bool ok = true;
       bool any = false;
       const int kc = Cfg::FOLD ? args.kchunk : (1 << 30);
@@ -654,6 +827,14 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
            t >= 0 && ok;
            t = next_tile<false>(args, t, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutMma)) {
         const int4 tile = args.tiles[t];
+        const uint32_t x0 = tmem_base + (uint32_t)(Cfg::CORR_COL + (nt & 1) * BN);
+        if (Cfg::SPLIT && tile.z < tile.w) {
+          if (!mbar_wait(&xempty[nt & 1], ((uint32_t)(nt >> 1) & 1u) ^ 1u, abort_flag, args.err, kDevErrTimeoutMma)) {
+            ok = false;
+            break;
+          }
+          ++nt;
+        }
         for (int c0 = tile.z; c0 < tile.w && ok; c0 += kc, ++it) {
           const int c1 = (tile.w - c0 > kc) ? c0 + kc : tile.w;
           const int buf = it & 1;
@@ -663,7 +844,7 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
             break;
           }
           tc_fence_after();
-          const uint32_t d0 = tmem_base + (uint32_t)(buf * Cfg::ACC_COLS);
+          const uint32_t d0 = tmem_base + (uint32_t)(buf * BN);
           for (int kb = c0; kb < c1; ++kb) {
             if (!mbar_wait(&full[s], ph, abort_flag, args.err, kDevErrTimeoutMma)) {
               ok = false;
@@ -681,11 +862,11 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
                 umma_f8(d0, da, db, Cfg::IDESC, acc);
               else
                 umma_f16(d0, da, db, Cfg::IDESC, acc);
-              if constexpr (Cfg::NSPLIT > 1) {
+              if constexpr (Cfg::SPLIT) {
                 const uint64_t da_lo = operand_desc<Cfg::A_MN>(a_hi + Cfg::A_BYTES, kk);
                 const uint64_t db_lo = operand_desc<Cfg::B_MN>(b_hi + Cfg::B_BYTES, kk);
-                umma_f16(d0 + BN, da, db_lo, Cfg::IDESC, acc);
-                umma_f16(d0 + BN, da_lo, db, Cfg::IDESC, 1u);
+                umma_f16(x0, da, db_lo, Cfg::IDESC, (kb > tile.z || kk > 0) ? 1u : 0u);
+                umma_f16(x0, da_lo, db, Cfg::IDESC, 1u);
               }
             }
             any = true;
@@ -712,15 +893,10 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
       }
     }
     __syncwarp();
-  } else if (Cfg::PF && warp == 6) {
-    // ------------------------------------------------------------ C loader (PF)
-    // Walks the CTA's tiles in the epilogue's chunk order; chunk n goes to
-    // ring slot n % C_SLOTS once the epilogue has given back the slot's
-    // previous chunk (n - C_SLOTS).
+  } else if (warp == 2) {
+    // ------------------------------------------------------------ C loader
     if (lane == 0) {
-      int slot = 0;
-      uint32_t ph = 0;
-      uint32_t armed = 0, armed_phase = 0;  // per-slot: a load was armed / its phase
+      CLoader<Cfg::C_SLOTS, Cfg::GROUP_BYTES / 4> ld(stage_c, cfull, cfree);
       bool ok = true;
       int tq = 0;
       uint32_t tq_ph = 0;
@@ -730,230 +906,34 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
            t = next_tile<false>(args, t, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutProducer)) {
         const int4 tile = args.tiles[t];
         const GemmArgs& P = tile_problem<GROUPED>(args, t);
-        if (!P.tma_c) continue;
-        const bool need = P.beta != 0.0f || tile_reaches_mask(P, tile.x, tile.y, BM, BN);
-        for (int c0 = 0; c0 < BN && tile.y + c0 < P.N; c0 += 32) {
-          if (!mbar_wait(&cfree[slot], ph ^ 1u, abort_flag, args.err, kDevErrTimeoutProducer)) {
-            ok = false;
-            break;
-          }
-          if (need) {
-            mbar_arrive_expect_tx(&cload[slot], Cfg::EPI_CHUNK_BYTES);
-            tma_load_2d(stage_c + slot * (128 * 32), &P.mapC, &cload[slot], tile.x, tile.y + c0);
-            armed |= 1u << slot;
-            armed_phase = (armed_phase & ~(1u << slot)) | (ph << slot);
-          } else {
-            // the slot's earlier load was consumed before the slot came back
-            armed &= ~(1u << slot);
-            mbar_arrive(&cload[slot]);
-          }
-          if (++slot == Cfg::C_SLOTS) {
-            slot = 0;
-            ph ^= 1u;
-          }
-        }
+        if (tile_staged(P, tile_reaches_mask(P, tile.x, tile.y, BM, BN)))
+          ok = ld.tile(P, tile.x, tile.y, Cfg::GC, abort_flag);
       }
-      // every armed load lands before the CTA exits (immediate unless the
-      // epilogue left early)
-      for (int i = 0; i < Cfg::C_SLOTS; ++i) {
-        if (!((armed >> i) & 1u)) continue;
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(&cload[i], (armed_phase >> i) & 1u))
-          if (globaltimer_ns() - t0 > 1000000000ull) {
-            if (args.err) atomicCAS(args.err, 0, kDevErrTimeoutTeardown);
-            break;
-          }
-      }
+      ld.drain(args.err);
     }
     __syncwarp();
-  } else {
+  } else if (warp >= kEpiWarp0) {
     // ------------------------------------------------------------ epilogue
     const int quarter = warp & 3;  // TMEM lane quarter this warp may access
-    const int row = quarter * 32 + lane;
-    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    const bool issuer = (warp == 2 && lane == 0);
-    EpiState es{0, 0u, false};
-    int it = 0;
-    bool ok = true;
+    const int group = (warp - kEpiWarp0) >> 2, gc0 = group * Cfg::GC;
+    const uint32_t tmem = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)gc0;
+    EpiGroup<Cfg::C_SLOTS, Cfg::SIDE> g{stage_c + group * (Cfg::GROUP_BYTES / 4), cfull + group * Cfg::C_SLOTS,
+                             cfree + group * Cfg::C_SLOTS, 1 + group, quarter * 32 + lane,
+                             quarter == 0 && lane == 0};
+    int it = 0, nt = 0;
     int tq = 0;
     uint32_t tq_ph = 0;
-    if constexpr (Cfg::PF) {
-      PfState pf{0, 0u, -1, 0};
-      __half* side_base = reinterpret_cast<__half*>(stage_c + Cfg::C_SLOTS * (128 * 32));
-      for (int t = next_tile<true>(args, -1, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutEpilogue);
-           t >= 0 && ok;
-           t = next_tile<true>(args, t, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutEpilogue)) {
-        const int4 tile = args.tiles[t];
-        const GemmArgs& P = tile_problem<GROUPED>(args, t);
-        const long long gi = (long long)tile.x + row;
-        const bool row_ok = gi < P.M;
-        const bool tile_masked = tile_reaches_mask(P, tile.x, tile.y, BM, BN);
-        const bool need_load = P.beta != 0.0f || tile_masked;
-        const StoreK sk(P);
-        if constexpr (!Cfg::FOLD) {
-          const int buf = it & 1;
-          const uint32_t tph = (uint32_t)(it >> 1) & 1u;
-          ++it;
-          const bool got = mbar_wait(&tfull[buf], tph, abort_flag, args.err, kDevErrTimeoutEpilogue);
-          if (named_bar_any(1, 128, !got)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t tacc = tmem_base + lane_addr + (uint32_t)(buf * Cfg::ACC_COLS);
-#pragma unroll 1
-          for (int c0 = 0; c0 < BN; c0 += 32) {
-            float v[32];
-            tmem_ld32(tacc + c0, v);
-            if (c0 == BN - 32) {
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&tempty[buf]);
-            }
-            if (tile.y + c0 >= P.N) continue;
-            if (P.tma_c) {
-              if (!epilogue_chunk_pf<Cfg::C_SLOTS>(P, stage_c, side_base, cload, cfree, pf, v, tile.x, tile.y + c0,
-                                                   row, need_load, issuer, abort_flag)) {
-                ok = false;
-                break;
-              }
-            } else if (row_ok)
-              epilogue_store32(sk, v, gi, (long long)tile.y + c0);
-          }
-        } else {
-          float acc[BN];
-#pragma unroll
-          for (int j = 0; j < BN; ++j) acc[j] = 0.f;
-          for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk) {
-            const int buf = it & 1;
-            const uint32_t tph = (uint32_t)(it >> 1) & 1u;
-            ++it;
-            const bool got = mbar_wait(&tfull[buf], tph, abort_flag, args.err, kDevErrTimeoutEpilogue);
-            if (named_bar_any(1, 128, !got)) {
-              ok = false;
-              break;
-            }
-            tc_fence_after();
-            const uint32_t tacc = tmem_base + lane_addr + (uint32_t)(buf * Cfg::ACC_COLS);
-#pragma unroll
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-              float v[32], w[32];
-              tmem_ld32x2(tacc + c0, tacc + BN + c0, v, w);
-#pragma unroll
-              for (int j = 0; j < 32; ++j) acc[c0 + j] += fmaf(args.corr_scale, w[j], v[j]);
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[buf]);
-          }
-          if (!ok) break;
-#pragma unroll
-          for (int c0 = 0; c0 < BN; c0 += 32) {
-            if (tile.y + c0 >= P.N) continue;
-            if (P.tma_c) {
-              if (!epilogue_chunk_pf<Cfg::C_SLOTS>(P, stage_c, side_base, cload, cfree, pf, acc + c0, tile.x,
-                                                   tile.y + c0, row, need_load, issuer, abort_flag)) {
-                ok = false;
-                break;
-              }
-            } else if (row_ok)
-              epilogue_store32(sk, acc + c0, gi, (long long)tile.y + c0);
-          }
-        }
-      }
-    } else
-    for (int t = next_tile<true>(args, -1, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutEpilogue);
-         t >= 0 && ok;
-         t = next_tile<true>(args, t, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutEpilogue)) {
+    for (int t = next_tile<true>(args, -1, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutEpilogue,
+                                 g.bar);
+         t >= 0; t = next_tile<true>(args, t, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag,
+                                     kDevErrTimeoutEpilogue, g.bar)) {
       const int4 tile = args.tiles[t];
       const GemmArgs& P = tile_problem<GROUPED>(args, t);
-      const long long gi = (long long)tile.x + row;
-      const bool row_ok = gi < P.M;
-      // the tile crosses the masked (upper) region: min(i - j) < diag
-      const bool tile_masked = tile_reaches_mask(P, tile.x, tile.y, BM, BN);
-      // masked tiles with beta == 0 store their unmasked elements directly:
-      // the TMA path would first have to load C to keep the masked ones
-      const bool direct = tile_masked && P.beta == 0.0f;
-      const StoreK sk(P);
-      if constexpr (!Cfg::FOLD) {
-        const int buf = it & 1;
-        const uint32_t tph = (uint32_t)(it >> 1) & 1u;
-        ++it;
-        // one decision for all 128 epilogue threads: the chunks below hold named barriers
-        if (named_bar_any(1, 128, !mbar_wait(&tfull[buf], tph, abort_flag, args.err, kDevErrTimeoutEpilogue)))
-          break;
-        tc_fence_after();
-        const uint32_t tacc = tmem_base + lane_addr + (uint32_t)(buf * Cfg::ACC_COLS);
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          float v[32];
-          tmem_ld32(tacc + c0, v);
-          if (c0 == BN - 32) {  // accumulator fully read: hand it back to the MMA warp
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[buf]);
-          }
-          if (P.tma_c && !direct) {
-            if (tile.y + c0 < P.N)
-              epilogue_chunk_tma(P, stage_c, cload, es, v, tile.x, tile.y + c0, row, P.beta != 0.0f || tile_masked,
-                                 issuer, abort_flag);
-          } else if (row_ok) {
-            epilogue_store32(sk, v, gi, (long long)tile.y + c0);
-          }
-        }
-      } else {
-        float acc[BN];
-#pragma unroll
-        for (int j = 0; j < BN; ++j) acc[j] = 0.f;
-        for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk) {
-          const int buf = it & 1;
-          const uint32_t tph = (uint32_t)(it >> 1) & 1u;
-          ++it;
-          if (named_bar_any(1, 128, !mbar_wait(&tfull[buf], tph, abort_flag, args.err, kDevErrTimeoutEpilogue))) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t tacc = tmem_base + lane_addr + (uint32_t)(buf * Cfg::ACC_COLS);
-          if constexpr (Cfg::FP8) {
-            // this round is K block c0k (kchunk = 1): scale by both blocks' scales
-            const int kbs = (P.k_off >> 7) + c0k;
-            const float sc = P.scale_a[(long long)((P.a_off + tile.x) >> 7) * P.scale_ld + kbs] *
-                             P.scale_b[(long long)((P.b_off + tile.y) >> 7) * P.scale_ld + kbs];
-#pragma unroll
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-              float v[32];
-              tmem_ld32(tacc + c0, v);
-#pragma unroll
-              for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(sc, v[j], acc[c0 + j]);
-            }
-          } else {
-#pragma unroll
-            for (int c0 = 0; c0 < BN; c0 += 32) {
-              float v[32], w[32];
-              tmem_ld32x2(tacc + c0, tacc + BN + c0, v, w);
-#pragma unroll
-              for (int j = 0; j < 32; ++j) acc[c0 + j] += fmaf(args.corr_scale, w[j], v[j]);
-            }
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[buf]);
-        }
-        if (!ok) break;
-#pragma unroll
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          if (P.tma_c && !direct) {
-            if (tile.y + c0 < P.N)
-              epilogue_chunk_tma(P, stage_c, cload, es, acc + c0, tile.x, tile.y + c0, row,
-                                 P.beta != 0.0f || tile_masked, issuer, abort_flag);
-          } else if (row_ok) {
-            epilogue_store32(sk, acc + c0, gi, (long long)tile.y + c0);
-          }
-        }
-      }
+      TileAcc<Cfg> acc{args, P, tile, gc0, tmem, tfull, tempty, xempty, it, nt, abort_flag};
+      const bool staged = tile_staged(P, tile_reaches_mask(P, tile.x, tile.y, BM, BN));
+      if (!epilogue_tile<Cfg::GC>(P, g, acc, tile.x, tile.y + gc0, staged, abort_flag)) break;
     }
-    if (issuer) bulk_wait<0>();  // all TMA stores complete before the CTA retires
+    if (g.issuer) bulk_wait<0>();  // all TMA stores complete before the CTA retires
   }
 
   tc_fence_before();
@@ -963,56 +943,71 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1) gemm_kernel(const __grid_cons
 }
 
 // ---------------------------------------------------------------------------
-// Pair variant (plain FP16): a cluster of two CTAs computes 256 x 256 output
-// tiles with tcgen05.mma.cta_group::2. CTA r of the pair loads rows
-// [m0 + 128r, +128) of A and rows [n0 + 128r, +128) of B (half of the tile's
-// columns) into its own shared memory; the leader (r = 0) issues the 256-row
-// MMA, which reads both CTAs' halves, and each CTA's TMEM receives its 128
-// accumulator rows. Per SM, one 64-deep K slab moves 32 KB from L2 instead of
-// the single-CTA tile's 48 KB for the same MMA work.
+// Pair variant: a cluster of two CTAs computes 256 x 256 output tiles with
+// tcgen05.mma.cta_group::2. CTA r of the pair loads rows [m0 + 128r, +128) of
+// A and rows [n0 + 128r, +128) of B (half of the tile's columns) into its own
+// shared memory; the leader (r = 0) issues the 256-row MMA, which reads both
+// CTAs' halves, and each CTA's TMEM receives its 128 accumulator rows. Per SM,
+// one 64-deep K slab moves 32 KB from L2 instead of the single-CTA tile's
+// 48 KB for the same MMA work.
 //   full[s]   leader only: both CTAs' loads complete_tx on it, the leader's
 //             producer arms it with both CTAs' bytes;
 //   empty[s]  both CTAs: the leader's commit multicasts to the pair;
 //   tfull[b]  both CTAs: the leader's commit multicasts to the pair;
-//   tempty[b] leader only: the 8 epilogue warps of the pair arrive remotely.
+//   tempty[b] leader only: the 16 epilogue warps of the pair arrive remotely.
 // Every wait is bounded like the single-CTA kernel's; a cluster barrier
 // before TMEM is freed keeps either CTA from leaving while the pair's MMAs
 // or remote arrivals may still touch it.
-// DIRECT: launches that read no C and write no side copies (beta = 0, e.g.
-// SYRK) store each thread's row of a chunk straight from registers (a
-// warp's 32 rows of a column are one 128-byte line), which frees the
-// epilogue's staging buffers for a seventh operand stage.
-// NSPLIT = 3 (split precision): 256 x 128 pair tiles with hi/lo operands
-// (each CTA loads 128 rows of A hi and lo and 64 rows of B hi and lo per K
-// block) and two accumulators per TMEM buffer, hi*hi and hi*lo + lo*hi;
-// the MMA issuer runs a tile's K range in rounds of kchunk K-blocks, one
-// TMEM buffer per round, and the epilogue folds each round into FP32
-// registers (acc += corr_scale * corr + main), as the single-CTA split
-// kernel does. Per SM and 16-deep K step the three MMAs read 6 KB of shared
-// memory each, against 8 KB for the single-CTA 128 x 128 split tile, which
-// is bound by shared-memory bandwidth.
-template <bool A_MN_, bool B_MN_, bool DIRECT_ = false, int NSPLIT_ = 1>
+//
+// kDirect: launches that read no C and write no side copies (beta = 0, e.g.
+// SYRK) store each thread's row of a chunk straight from registers (a warp's
+// 32 rows of one column are one 128-byte line), which frees the C slots for
+// more operand stages. kStaged: the others, with a ring of C slots.
+// kSplit: hi/lo operands, three products (64 KB a stage). Main and correction
+// accumulators take all 512 TMEM columns, so nothing is double-buffered;
+// instead each K-block runs its four main MMAs before its eight correction
+// MMAs: while a round's last correction MMAs run (1024 cycles per SM), the
+// epilogue reads the main accumulator, and the next round's main MMAs find it
+// free. Buffer 0 is the main accumulator (one phase a round), buffer 1 the
+// correction (one phase a tile). Per 64-deep K block and SM the 256 x 256 tile
+// moves 64 KB into shared memory and 96 KB out of it for 1536 MMA cycles,
+// where 256 x 128 tiles (which left room to double-buffer) moved 96 + 144 KB
+// and kept the tensor pipe 65 % busy: SYR2K n = 16384, k = 4096 went from 6.0
+// to 5.3 ms.
+// kFp8: e4m3 operands, one 128-deep K block a round (512 MMA cycles per SM),
+// the accumulators double-buffered and folded with the blocks' scales. The
+// fold, not the MMAs, bounds the round; single-CTA 128 x 128 tiles have 256 MMA
+// cycles a round and as long a fold for a quarter of the work a pair does:
+// SYMM 16384 went from 8.8 to 6.6 ms.
+// The fold modes keep 128 sums per epilogue thread: the first four warps give
+// registers to the epilogue's eight (setmaxnreg: 128 x 72 + 256 x 216 = 384 x
+// 168, the launch's allocation).
+enum class PairMode { kStaged, kDirect, kSplit, kFp8 };
+
+template <bool A_MN_, bool B_MN_, PairMode MODE_>
 struct PairCfg {
-  static constexpr int NSPLIT = NSPLIT_;
-  static constexpr bool FOLD = NSPLIT > 1;
-  static constexpr int NOPS = FOLD ? 2 : 1;  // copies per operand (hi[, lo])
-  static constexpr int NACC = FOLD ? 2 : 1;  // accumulators per TMEM buffer
-  static constexpr int BM = 128, BN = FOLD ? 128 : 256, BK = 64;  // BM: rows per CTA; BN: the pair tile's columns
+  static constexpr PairMode MODE = MODE_;
+  static constexpr bool SPLIT = MODE == PairMode::kSplit, FP8 = MODE == PairMode::kFp8;
+  static constexpr bool FOLD = SPLIT || FP8, DIRECT = MODE == PairMode::kDirect;
+  static constexpr int NOPS = SPLIT ? 2 : 1;  // copies per operand (hi[, lo])
+  static constexpr int ELEM = FP8 ? 1 : 2;
+  static constexpr int BM = 128, BN = 256, BK = 128 / ELEM;  // BM: rows per CTA; BN: the pair tile's columns
   static constexpr bool A_MN = A_MN_, B_MN = B_MN_;
-  static constexpr bool DIRECT = DIRECT_;
-  static_assert(!(FOLD && DIRECT), "the split pair tile stages its epilogue");
-  static constexpr int A_BYTES = BM * BK * 2;
-  static constexpr int B_BYTES = (BN / 2) * BK * 2;
+  static constexpr int A_BYTES = BM * BK * ELEM;
+  static constexpr int B_BYTES = (BN / 2) * BK * ELEM;
   static constexpr int STAGE_BYTES = NOPS * (A_BYTES + B_BYTES);
-  static constexpr int STAGES = FOLD ? 4 : (DIRECT ? 7 : 6);
-  static constexpr int ACC_COLS = NACC * BN;
-  static constexpr int TMEM_COLS = 2 * ACC_COLS;
-  static_assert(TMEM_COLS <= 512, "TMEM budget");
-  static constexpr int EPI_BYTES = DIRECT ? 0 : 2 * 128 * 32 * 4;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + 256;
+  static constexpr int STAGES = SPLIT ? 3 : (FP8 ? 6 : (DIRECT ? 7 : 5));
+  static constexpr int TMEM_COLS = 512;
+  static constexpr int GC = BN / kEpiGroups;
+  static constexpr int CHUNK_BYTES = 128 * kEpiCols * 4;
+  static constexpr int C_SLOTS = DIRECT ? 0 : (FOLD ? 2 : 4), SIDE = 0;  // per group
+  static constexpr int GROUP_BYTES = (C_SLOTS + SIDE) * CHUNK_BYTES;
+  static constexpr int EPI_BYTES = kEpiGroups * GROUP_BYTES;
+  static constexpr int BAR_BYTES = 320;
+  static_assert(8 * (2 * STAGES + 5 + 2 * kEpiGroups * C_SLOTS) + 8 <= BAR_BYTES, "barrier space");
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + BAR_BYTES;
   static_assert(SMEM_BYTES <= 232448, "shared memory budget");
   static constexpr uint32_t IDESC = idesc_f16(2 * BM, BN, false, A_MN, B_MN);
-  static constexpr int THREADS = 192;
 };
 
 template <bool MN, int ROWS>
@@ -1026,10 +1021,100 @@ __device__ __forceinline__ void load_operand_pair(uint8_t* dst, const CUtensorMa
   }
 }
 
+// Accumulators of one pair tile, as an epilogue warp of CTA `rank` sees them.
 template <class Cfg>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+struct PairAcc {
+  static constexpr bool kEarlyLoad = !Cfg::FOLD;
+  const GemmArgs& args;
+  int4 tile;
+  int m0, gc0;
+  uint32_t tmem;
+  uint64_t* tfull;
+  uint32_t tempty_leader;
+  int &it, &nt;
+  volatile int* abort_flag;
+  float acc[Cfg::FOLD ? Cfg::GC : 16];
+  int buf = 0;
+
+  __device__ __forceinline__ bool wait(int b, uint32_t ph) {
+    const bool got = mbar_wait(&tfull[b], ph, abort_flag, args.err, kDevErrTimeoutEpilogue);
+    tc_fence_after();
+    return __all_sync(0xffffffffu, got);  // one decision per warp: TMEM loads follow
+  }
+  // this CTA's warp has read its part of buffer b: tell the leader
+  __device__ __forceinline__ void release(int b) {
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive_cluster(tempty_leader + 8u * (uint32_t)b);
+  }
+  __device__ __forceinline__ bool begin() {
+    if constexpr (!Cfg::FOLD) {
+      buf = it & 1;
+      const uint32_t ph = (uint32_t)(it >> 1) & 1u;
+      ++it;
+      return wait(buf, ph);
+    } else {
+#pragma unroll
+      for (int j = 0; j < Cfg::GC; ++j) acc[j] = 0.f;
+      if constexpr (Cfg::FP8) {
+        Fp8Scales sc(args, m0, tile.y + gc0, tile.z, tile.w);
+        for (int kb = tile.z; kb < tile.w; ++kb, ++it) {
+          const float s = sc.next(kb, tile.w);
+          const int b = it & 1;
+          if (!wait(b, (uint32_t)(it >> 1) & 1u)) return false;
+          const uint32_t ta = tmem + (uint32_t)(b * Cfg::BN);
+#pragma unroll
+          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
+            float v[32];
+            tmem_ld32(ta + c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(s, v[j], acc[c0 + j]);
+          }
+          release(b);
+        }
+      } else {
+        for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk, ++it) {
+          if (!wait(0, (uint32_t)it & 1u)) return false;
+#pragma unroll
+          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
+            float v[32];
+            tmem_ld32(tmem + c0, v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
+          }
+          release(0);
+        }
+        if (tile.z < tile.w) {
+          if (!wait(1, (uint32_t)nt & 1u)) return false;
+          ++nt;
+#pragma unroll
+          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
+            float w[32];
+            tmem_ld32(tmem + Cfg::BN + c0, w);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(args.corr_scale, w[j], acc[c0 + j]);
+          }
+          release(1);
+        }
+      }
+      return true;
+    }
+  }
+  __device__ __forceinline__ void chunk(int c, float* v) {
+    if constexpr (Cfg::FOLD) {
+      pick16(acc, c, v);
+    } else {
+      tmem_ld16(tmem + (uint32_t)(buf * Cfg::BN + c * kEpiCols), v);
+      if (c == Cfg::GC / kEpiCols - 1) release(buf);
+    }
+  }
+};
+
+template <class Cfg>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     gemm_pair_kernel(const __grid_constant__ GemmArgs args) {
   constexpr int BN = Cfg::BN, BK = Cfg::BK, STAGES = Cfg::STAGES;
+  constexpr int kSlots = kEpiGroups * Cfg::C_SLOTS;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* stage_c = reinterpret_cast<float*>(smem + STAGES * Cfg::STAGE_BYTES);
@@ -1038,8 +1123,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   uint64_t* tfull = empty + STAGES;  // [2]
   uint64_t* tempty = tfull + 2;      // [2]
   uint64_t* drain = tempty + 2;      // [1]
-  uint64_t* cload = drain + 1;       // [2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cload + 2);
+  uint64_t* cfull = drain + 1;       // [group][C_SLOTS]
+  uint64_t* cfree = cfull + kSlots;  // [group][C_SLOTS]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cfree + kSlots);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -1055,8 +1141,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 8);
-      mbar_init(&cload[b], 1);
+      mbar_init(&tempty[b], 2 * 4 * kEpiGroups);
+    }
+    for (int b = 0; b < kSlots; ++b) {
+      mbar_init(&cfull[b], 1);
+      mbar_init(&cfree[b], 1);
     }
     mbar_init(drain, 1);
     *abort_flag = 0;
@@ -1065,6 +1154,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   if (warp == 0 && lane == 0) {
     tma_prefetch_map(&args.mapA[0]);
     tma_prefetch_map(&args.mapB[0]);
+    if (Cfg::NOPS > 1) {
+      tma_prefetch_map(&args.mapA[1]);
+      tma_prefetch_map(&args.mapB[1]);
+    }
     if (args.tma_c) tma_prefetch_map(&args.mapC);
   }
   if (warp == 1) {
@@ -1081,224 +1174,180 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
   const uint32_t full_leader = mapa_shared(smem_u32(full), 0);
   const uint32_t tempty_leader = mapa_shared(smem_u32(tempty), 0);
 
-  if (warp == 0) {
-    // ------------------------------------------------------------ producers (both CTAs)
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      uint32_t issued_mask = 0, phase_mask = 0;
-      bool ok = true;
-      for (int t = static_first(args, pair); t >= 0 && ok; t = static_next(args, pair, npairs, t)) {
-        if (debug_stall_tile(args.err, t)) break;  // test hook: this tile's loads never come
-        const int4 tile = args.tiles[t];
-        for (int kb = tile.z; kb < tile.w; ++kb) {
-          if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag, args.err, kDevErrTimeoutProducer)) {
-            ok = false;
-            break;
-          }
-          if (leader) mbar_arrive_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
-          uint8_t* st = smem + s * Cfg::STAGE_BYTES;
-          const int k = args.k_off + kb * BK;
-          const uint32_t bar = full_leader + 8u * (uint32_t)s;
-#pragma unroll
-          for (int h = 0; h < Cfg::NOPS; ++h) {
-            load_operand_pair<Cfg::A_MN, 128>(st + h * Cfg::A_BYTES, &args.mapA[h], bar,
-                                              args.a_off + tile.x + 128 * (int)rank, k);
-            load_operand_pair<Cfg::B_MN, BN / 2>(st + Cfg::NOPS * Cfg::A_BYTES + h * Cfg::B_BYTES, &args.mapB[h], bar,
-                                                 args.b_off + tile.y + (BN / 2) * (int)rank, k);
-          }
-          issued_mask |= 1u << s;
-          phase_mask = (phase_mask & ~(1u << s)) | (ph << s);
-          if (++s == STAGES) {
-            s = 0;
-            ph ^= 1u;
-          }
-        }
-      }
-      if (!ok) {
-        // Abort path: the leader sees its loads land on its own barriers; the
-        // peer's loads report to the leader, so the peer waits a bounded time.
-        if (leader) {
-          for (int i = 0; i < STAGES; ++i) {
-            if (!((issued_mask >> i) & 1u)) continue;
-            const uint64_t t0 = globaltimer_ns();
-            while (!mbar_try_wait(&full[i], (phase_mask >> i) & 1u))
-              if (globaltimer_ns() - t0 > 1000000000ull) break;
-          }
-        } else {
-          const uint64_t t0 = globaltimer_ns();
-          while (globaltimer_ns() - t0 < 2000000ull) {
-          }
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (leader)
-    if (leader && lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      int it = 0;
-      bool ok = true, any = false;
-      // a tile's K range in rounds of kchunk K-blocks (split) or one round
-      const int kc = Cfg::FOLD ? args.kchunk : (1 << 30);
-      for (int t = static_first(args, pair); t >= 0 && ok; t = static_next(args, pair, npairs, t)) {
-        const int4 tile = args.tiles[t];
-        for (int c0 = tile.z; c0 < tile.w && ok; c0 += kc, ++it) {
-          const int c1 = (tile.w - c0 > kc) ? c0 + kc : tile.w;
-          const int buf = it & 1;
-          const uint32_t tph = (uint32_t)(it >> 1) & 1u;
-          if (!mbar_wait(&tempty[buf], tph ^ 1u, abort_flag, args.err, kDevErrTimeoutMma)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t d0 = tmem_base + (uint32_t)(buf * Cfg::ACC_COLS);
-          for (int kb = c0; kb < c1; ++kb) {
-            if (!mbar_wait(&full[s], ph, abort_flag, args.err, kDevErrTimeoutMma)) {
+  if (warp < kEpiWarp0) {
+    if constexpr (Cfg::FOLD) setmaxnreg_dec<72>();
+    if (warp == 0) {
+      // ---------------------------------------------------------- producers (both CTAs)
+      if (lane == 0) {
+        int s = 0;
+        uint32_t ph = 0;
+        uint32_t issued_mask = 0, phase_mask = 0;
+        bool ok = true;
+        for (int t = static_first(args, pair); t >= 0 && ok; t = static_next(args, pair, npairs, t)) {
+          if (debug_stall_tile(args.err, t)) break;  // test hook: this tile's loads never come
+          const int4 tile = args.tiles[t];
+          for (int kb = tile.z; kb < tile.w; ++kb) {
+            if (!mbar_wait(&empty[s], ph ^ 1u, abort_flag, args.err, kDevErrTimeoutProducer)) {
               ok = false;
               break;
             }
-            tc_fence_after();
-            const uint32_t a = smem_u32(smem + s * Cfg::STAGE_BYTES), b = a + Cfg::NOPS * Cfg::A_BYTES;
+            if (leader) mbar_arrive_expect_tx(&full[s], 2 * Cfg::STAGE_BYTES);
+            uint8_t* st = smem + s * Cfg::STAGE_BYTES;
+            const int k = args.k_off + kb * BK;
+            const uint32_t bar = full_leader + 8u * (uint32_t)s;
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-              const uint32_t acc = (kb > c0 || kk > 0) ? 1u : 0u;
-              const uint64_t da = operand_desc<Cfg::A_MN>(a, kk), db = operand_desc<Cfg::B_MN>(b, kk);
-              umma_f16_pair(d0, da, db, Cfg::IDESC, acc);
-              if constexpr (Cfg::FOLD) {
-                umma_f16_pair(d0 + BN, da, operand_desc<Cfg::B_MN>(b + Cfg::B_BYTES, kk), Cfg::IDESC, acc);
-                umma_f16_pair(d0 + BN, operand_desc<Cfg::A_MN>(a + Cfg::A_BYTES, kk), db, Cfg::IDESC, 1u);
-              }
+            for (int h = 0; h < Cfg::NOPS; ++h) {
+              load_operand_pair<Cfg::A_MN, 128>(st + h * Cfg::A_BYTES, &args.mapA[h], bar,
+                                                args.a_off + tile.x + 128 * (int)rank, k);
+              load_operand_pair<Cfg::B_MN, BN / 2>(st + Cfg::NOPS * Cfg::A_BYTES + h * Cfg::B_BYTES, &args.mapB[h],
+                                                   bar, args.b_off + tile.y + (BN / 2) * (int)rank, k);
             }
-            any = true;
-            tc_commit_pair(&empty[s], 3);
+            issued_mask |= 1u << s;
+            phase_mask = (phase_mask & ~(1u << s)) | (ph << s);
             if (++s == STAGES) {
               s = 0;
               ph ^= 1u;
             }
           }
-          if (!ok) break;
-          tc_commit_pair(&tfull[buf], 3);
         }
-      }
-      if (!ok && any) {
-        tc_commit_pair(drain, 1);
-        const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(drain, 0)) {
-          if (globaltimer_ns() - t0 > 1000000000ull) {
-            if (args.err) atomicCAS(args.err, 0, kDevErrTimeoutTeardown);
-            break;
+        if (!ok) {
+          // Abort path: the leader sees its loads land on its own barriers; the
+          // peer's loads report to the leader, so the peer waits a bounded time.
+          if (leader) {
+            for (int i = 0; i < STAGES; ++i) {
+              if (!((issued_mask >> i) & 1u)) continue;
+              const uint64_t t0 = globaltimer_ns();
+              while (!mbar_try_wait(&full[i], (phase_mask >> i) & 1u))
+                if (globaltimer_ns() - t0 > 1000000000ull) break;
+            }
+          } else {
+            const uint64_t t0 = globaltimer_ns();
+            while (globaltimer_ns() - t0 < 2000000ull) {
+            }
           }
         }
       }
+      __syncwarp();
+    } else if (warp == 1) {
+      // ---------------------------------------------------------- MMA issuer (leader)
+      if (leader && lane == 0) {
+        int s = 0;
+        uint32_t ph = 0;
+        int it = 0, nt = 0;  // rounds and (split) tiles: buffers and phases, as in gemm_kernel
+        bool ok = true, any = false;
+        const int kc = Cfg::FOLD ? args.kchunk : (1 << 30);
+        for (int t = static_first(args, pair); t >= 0 && ok; t = static_next(args, pair, npairs, t)) {
+          const int4 tile = args.tiles[t];
+          for (int c0 = tile.z; c0 < tile.w && ok; c0 += kc, ++it) {
+            const int c1 = (tile.w - c0 > kc) ? c0 + kc : tile.w;
+            const int buf = Cfg::SPLIT ? 0 : (it & 1);
+            const uint32_t tph = (uint32_t)(Cfg::SPLIT ? it : (it >> 1)) & 1u;
+            if (!mbar_wait(&tempty[buf], tph ^ 1u, abort_flag, args.err, kDevErrTimeoutMma)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t d0 = tmem_base + (uint32_t)(buf * BN);
+            for (int kb = c0; kb < c1; ++kb) {
+              if (!mbar_wait(&full[s], ph, abort_flag, args.err, kDevErrTimeoutMma)) {
+                ok = false;
+                break;
+              }
+              tc_fence_after();
+              const uint32_t a = smem_u32(smem + s * Cfg::STAGE_BYTES), b = a + Cfg::NOPS * Cfg::A_BYTES;
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk) {
+                const uint32_t acc = (kb > c0 || kk > 0) ? 1u : 0u;
+                const uint64_t da = operand_desc<Cfg::A_MN>(a, kk), db = operand_desc<Cfg::B_MN>(b, kk);
+                if constexpr (Cfg::FP8)
+                  umma_f8_pair(d0, da, db, Cfg::IDESC, acc);
+                else
+                  umma_f16_pair(d0, da, db, Cfg::IDESC, acc);
+              }
+              any = true;
+              if constexpr (Cfg::SPLIT) {
+                if (kb == c1 - 1) tc_commit_pair(&tfull[0], 3);  // the round's main products are issued
+                if (kb == tile.z) {
+                  if (!mbar_wait(&tempty[1], ((uint32_t)nt & 1u) ^ 1u, abort_flag, args.err, kDevErrTimeoutMma)) {
+                    ok = false;
+                    break;
+                  }
+                  tc_fence_after();
+                }
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                  const uint64_t da = operand_desc<Cfg::A_MN>(a, kk), db = operand_desc<Cfg::B_MN>(b, kk);
+                  umma_f16_pair(d0 + BN, da, operand_desc<Cfg::B_MN>(b + Cfg::B_BYTES, kk), Cfg::IDESC,
+                                (kb > tile.z || kk > 0) ? 1u : 0u);
+                  umma_f16_pair(d0 + BN, operand_desc<Cfg::A_MN>(a + Cfg::A_BYTES, kk), db, Cfg::IDESC, 1u);
+                }
+              }
+              tc_commit_pair(&empty[s], 3);
+              if (++s == STAGES) {
+                s = 0;
+                ph ^= 1u;
+              }
+            }
+            if (!ok) break;
+            if constexpr (!Cfg::SPLIT) tc_commit_pair(&tfull[buf], 3);
+          }
+          if (!ok) break;
+          if constexpr (Cfg::SPLIT) {
+            if (tile.z < tile.w) {
+              tc_commit_pair(&tfull[1], 3);
+              ++nt;
+            }
+          }
+        }
+        if (!ok && any) {
+          tc_commit_pair(drain, 1);
+          const uint64_t t0 = globaltimer_ns();
+          while (!mbar_try_wait(drain, 0)) {
+            if (globaltimer_ns() - t0 > 1000000000ull) {
+              if (args.err) atomicCAS(args.err, 0, kDevErrTimeoutTeardown);
+              break;
+            }
+          }
+        }
+      }
+      __syncwarp();
+    } else if (!Cfg::DIRECT && warp == 2) {
+      // ---------------------------------------------------------- C loader (both CTAs)
+      if constexpr (!Cfg::DIRECT) {
+        if (lane == 0) {
+          CLoader<Cfg::C_SLOTS, Cfg::GROUP_BYTES / 4> ld(stage_c, cfull, cfree);
+          bool ok = true;
+          for (int t = static_first(args, pair); t >= 0 && ok; t = static_next(args, pair, npairs, t)) {
+            const int4 tile = args.tiles[t];
+            const int m0 = tile.x + 128 * (int)rank;
+            if (m0 < args.M && tile_staged(args, tile_reaches_mask(args, m0, tile.y, 128, BN)))
+              ok = ld.tile(args, m0, tile.y, Cfg::GC, abort_flag);
+          }
+          ld.drain(args.err);
+        }
+        __syncwarp();
+      }
     }
-    __syncwarp();
   } else {
     // ------------------------------------------------------------ epilogue (both CTAs)
+    if constexpr (Cfg::FOLD) setmaxnreg_inc<216>();
     const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    const bool issuer = (warp == 2 && lane == 0);
-    const bool c_prefetch = args.c_ahead != 0;
-    EpiState es{0, 0u, false};
-    int it = 0;
+    const int group = (warp - kEpiWarp0) >> 2, gc0 = group * Cfg::GC;
+    const uint32_t tmem = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)gc0;
+    EpiGroup<Cfg::C_SLOTS, Cfg::SIDE> g{stage_c + group * (Cfg::GROUP_BYTES / 4), cfull + group * Cfg::C_SLOTS,
+                             cfree + group * Cfg::C_SLOTS, 1 + group, quarter * 32 + lane,
+                             quarter == 0 && lane == 0};
+    int it = 0, nt = 0;
     for (int t = static_first(args, pair); t >= 0; t = static_next(args, pair, npairs, t)) {
       const int4 tile = args.tiles[t];
       const int m0 = tile.x + 128 * (int)rank;
-      const long long gi = (long long)m0 + row;
-      const bool row_ok = gi < args.M;
-      const bool tile_masked = tile_reaches_mask(args, m0, tile.y, 128, BN);
-      const bool direct = tile_masked && args.beta == 0.0f;  // as in the single-CTA kernel
-      const StoreK sk(args);
-      // C loads one chunk ahead (the first before the accumulator wait) for
-      // tiles that read C and stage no side copies in shared memory
-      const long long nrem = ((long long)args.N - tile.y + 31) / 32;
-      const int nval = nrem < BN / 32 ? (int)nrem : BN / 32;
-      const bool ahead = !Cfg::DIRECT && c_prefetch && args.tma_c && !direct && m0 < args.M &&
-                         (args.beta != 0.0f || tile_masked) &&
-                         !(args.tma_out && m0 < args.out_m && tile.y < args.out_n);
-      const int b0 = es.chunk & 1;
-      const uint32_t ph0 = (es.lphase >> b0) & 1u;
-      // one 128 x 32 chunk of this CTA's output rows: alpha * v (+ beta * C)
-      auto store_chunk = [&](const float* v, int c0) {
-        if (ahead) {
-          if (c0 / 32 < nval) {
-            if (issuer && c0 / 32 + 1 < nval) c_issue_load(args, stage_c, cload, es, 1, m0, tile.y + c0 + 32);
-            epilogue_chunk_loaded(args, stage_c, cload, es, v, m0, tile.y + c0, row, issuer, abort_flag);
-          }
-        } else if (!Cfg::DIRECT && args.tma_c && !direct) {
-          if (tile.y + c0 < args.N && m0 < args.M)
-            epilogue_chunk_tma(args, stage_c, cload, es, v, m0, tile.y + c0, row, args.beta != 0.0f || tile_masked,
-                               issuer, abort_flag);
-        } else if (row_ok) {
-          epilogue_store32(sk, v, gi, (long long)tile.y + c0);
-        }
-      };
-      // the chunk-0 load in flight lands before the CTA leaves (bounded)
-      auto drain_ahead = [&]() {
-        if (ahead && issuer) {
-          const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(&cload[b0], ph0))
-            if (globaltimer_ns() - t0 > 1000000000ull) break;
-        }
-      };
-      if (ahead && issuer) c_issue_load(args, stage_c, cload, es, 0, m0, tile.y);
-      if constexpr (Cfg::FOLD) {
-        float acc[BN];
-#pragma unroll
-        for (int j = 0; j < BN; ++j) acc[j] = 0.f;
-        bool bad = false;
-        for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk, ++it) {
-          const int buf = it & 1;
-          const uint32_t tph = (uint32_t)(it >> 1) & 1u;
-          if (named_bar_any(1, 128, !mbar_wait(&tfull[buf], tph, abort_flag, args.err, kDevErrTimeoutEpilogue))) {
-            bad = true;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t tacc = tmem_base + lane_addr + (uint32_t)(buf * Cfg::ACC_COLS);
-#pragma unroll
-          for (int c0 = 0; c0 < BN; c0 += 32) {
-            float v[32], w[32];
-            tmem_ld32x2(tacc + c0, tacc + BN + c0, v, w);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c0 + j] += fmaf(args.corr_scale, w[j], v[j]);
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(tempty_leader + 8u * (uint32_t)buf);
-        }
-        if (bad) {
-          drain_ahead();
-          break;
-        }
-#pragma unroll
-        for (int c0 = 0; c0 < BN; c0 += 32) store_chunk(acc + c0, c0);
-      } else {
-        const int buf = it & 1;
-        const uint32_t tph = (uint32_t)(it >> 1) & 1u;
-        ++it;
-        if (named_bar_any(1, 128, !mbar_wait(&tfull[buf], tph, abort_flag, args.err, kDevErrTimeoutEpilogue))) {
-          drain_ahead();
-          break;
-        }
-        tc_fence_after();
-        const uint32_t tacc = tmem_base + lane_addr + (uint32_t)(buf * Cfg::ACC_COLS);
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          float v[32];
-          tmem_ld32(tacc + c0, v);
-          if (c0 == BN - 32) {  // this CTA's half of the accumulator is read: tell the leader
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(tempty_leader + 8u * (uint32_t)buf);
-          }
-          store_chunk(v, c0);
-        }
-      }
+      PairAcc<Cfg> acc{args, tile, m0, gc0, tmem, tfull, tempty_leader, it, nt, abort_flag};
+      // rows wholly outside C are stored by neither path
+      const bool staged = !Cfg::DIRECT && m0 < args.M &&
+                          tile_staged(args, tile_reaches_mask(args, m0, tile.y, 128, BN));
+      if (!epilogue_tile<Cfg::GC>(args, g, acc, m0, tile.y + gc0, staged, abort_flag)) break;
     }
-    if (issuer) bulk_wait<0>();
+    if (g.issuer) bulk_wait<0>();
   }
 
   tc_fence_before();

@@ -120,6 +120,7 @@ struct GemmCall {
   // blocks of 128, per-(128-row block, K block) scales (row-block-major,
   // scale_ld K blocks per row block); tiles 128 x 128.
   bool pair = false;  // set by gemm_launch_plan: 256 x 256 tiles on CTA pairs (cta_group::2)
+  int epi_cols = 32;  // columns of the TMA boxes the epilogue moves C and the side copies in
   bool fp8 = false;
   const float* scale_a = nullptr;
   const float* scale_b = nullptr;
@@ -138,7 +139,7 @@ constexpr int kGemmBNFp8 = 128;  // FP8 tiles: 128 x 128, K blocks of 128
 int gemm_bn(Split s);
 int gemm_bn(Split s, int kblocks);
 
-tb_status gemm_launch(const GemmCall& call, cudaStream_t stream);
+tb_status gemm_launch(GemmCall& call, cudaStream_t stream);
 // GEMM engine for the large plain launches of this thread: -1 the default
 // (CTA pairs unless TB_GEMM_PAIR=0), 0 single-CTA 128 x 256 tiles, 1 CTA
 // pairs (256 x 256), 2 single-CTA 128 x 128 tiles (kEngineNarrow: twice the

@@ -170,7 +170,7 @@ __device__ __forceinline__ void dag_chunk(const GemmArgs& P, const StoreK& sk, f
       S[j * 128 + row] = r[j];
     }
   }
-  if (side_tile && gi < sk.out_m && gj0 < sk.out_n) store_fp16_copies(sk, r, gi, gj0);
+  if (side_tile && gi < sk.out_m && gj0 < sk.out_n) store_fp16_copies<32>(sk, r, gi, gj0);
   fence_proxy_async_smem();
   named_bar_sync(1, 128);
   if (issuer) {
@@ -366,6 +366,9 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
         const DagTask task = args.tasks[t];
         const bool split = task.meta.y != 0;
         const int kc = split ? args.kchunk : (1 << 30);
+        // split tasks: the correction stays in the upper half of the first
+        // round's buffer over all rounds (later rounds use lower halves only)
+        const uint32_t x0 = tmem_base + (uint32_t)((it & 1) * 256 + 128);
         for (int c0 = task.tile.z; c0 < task.tile.w && ok; c0 += kc, ++it) {
           const int c1 = (task.tile.w - c0 > kc) ? c0 + kc : task.tile.w;
           const int buf = it & 1;
@@ -404,8 +407,8 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
                 const uint64_t da_lo = operand_desc<A_MN>(st + kDagABytes, kk);
                 const uint64_t db_lo = operand_desc<B_MN>(st_lo, kk);
                 umma_f16(d0, da, db, IDESC_SPLIT, acc);
-                umma_f16(d0 + 128, da, db_lo, IDESC_SPLIT, acc);
-                umma_f16(d0 + 128, da_lo, db, IDESC_SPLIT, 1u);
+                umma_f16(x0, da, db_lo, IDESC_SPLIT, (kb > task.tile.z || kk > 0) ? 1u : 0u);
+                umma_f16(x0, da_lo, db, IDESC_SPLIT, 1u);
               } else {
                 umma_f16(d0, da, operand_desc<B_MN>(st + kDagABytes, kk), IDESC_PLAIN, acc);
               }
@@ -507,6 +510,16 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
         float acc[128];
 #pragma unroll
         for (int j = 0; j < 128; ++j) acc[j] = 0.f;
+        // main sums every round; the correction (upper half of the first
+        // round's buffer) once at the end. The buffers of the last two rounds
+        // go back together after that: one of them holds the correction.
+        const uint32_t xacc = tmem_base + lane_addr + (uint32_t)((it & 1) * 256 + 128);
+        int held = -1;
+        auto give_back = [&](int b) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&tempty[b]);
+        };
         for (int c0k = task.tile.z; c0k < task.tile.w; c0k += args.kchunk) {
           const int buf = it & 1;
           const uint32_t tph = (uint32_t)(it >> 1) & 1u;
@@ -519,14 +532,27 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
           const uint32_t tacc = tmem_base + lane_addr + (uint32_t)(buf * 256);
 #pragma unroll
           for (int c0 = 0; c0 < 128; c0 += 32) {
-            float v[32], w[32];
-            tmem_ld32x2(tacc + c0, tacc + 128 + c0, v, w);
+            float v[32];
+            tmem_ld32(tacc + c0, v);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c0 + j] += fmaf(P.corr_scale, w[j], v[j]);
+            for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
           }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[buf]);
+          const int left = task.tile.w - c0k;  // K-blocks from this round on
+          if (left <= args.kchunk) {           // the last round: every product is in
+#pragma unroll
+            for (int c0 = 0; c0 < 128; c0 += 32) {
+              float w[32];
+              tmem_ld32(xacc + c0, w);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(P.corr_scale, w[j], acc[c0 + j]);
+            }
+            if (held >= 0) give_back(held);
+            give_back(buf);
+          } else if (left <= 2 * args.kchunk) {
+            held = buf;
+          } else {
+            give_back(buf);
+          }
         }
         if (!ok) break;
         const StoreK sk(P);
@@ -1023,7 +1049,7 @@ tb_status trsm_solve_dag(TrsmCtx& c, const std::vector<long>& leaf_start, float*
   // every output (B and the FP16 side copies) must leave through TMA stores,
   // whose completion a tile waits for before it publishes its progress
   for (size_t i = 0; i < ops.size(); ++i)
-    if (!hops[i].tma_c || (ops[i].call.out_hi && !hops[i].tma_out))
+    if (!hops[i].tma_c)
       return trsm_solve_launches(c, leaf_start, B, ldb, rows, cols);
   const int4* d_tasks = upload_tiles(plan.packed, c.st);
   if (!d_tasks) return TB_ERROR_ALLOC;
