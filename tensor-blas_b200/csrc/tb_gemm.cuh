@@ -54,7 +54,6 @@ struct GemmArgs {
   CUtensorMap mapA[2];  // [0] hi, [1] lo (split mode only)
   CUtensorMap mapB[2];
   CUtensorMap mapC;     // fp32 C, box {128, 16} (TMA epilogue only)
-  CUtensorMap mapOut[2];  // fp16 side copies hi / lo over [0,out_m) x [0,out_n), box {128, 16}
   const int4* tiles;    // {m0, n0, kb_begin, kb_end}; m0/n0 relative to C
   int num_tiles;
   int a_off;  // row offset of the A operand in mapA's row coordinate
@@ -76,7 +75,6 @@ struct GemmArgs {
   long long ld_out;
   float out_lo_scale;
   int out_m, out_n;  // side copies only for rows < out_m and columns < out_n
-  int tma_out;       // 1: side copies through mapOut where they are staged (requires tma_c and tri == 0)
   int* err;
   // FP8: per-(128-row block, 128-deep K block) scales of the A and B
   // operands, row-block-major with scale_ld K blocks per row block.
@@ -169,9 +167,8 @@ constexpr int kGemmThreads = 32 * (kEpiWarp0 + 4 * kEpiGroups);
 
 // Shared memory left beside the operand stages goes to the C slots: a group's
 // loader ring runs that many 8 KB chunks ahead of its epilogue.
-// PF variants serve launches whose tiles have few K-blocks: there the
-// epilogue, not the MMA, bounds the tile, so they trade operand stages for C
-// slots and for staging buffers of the fp16 side copies.
+// PF variants serve launches whose tiles have few K-blocks: there C, not the
+// MMA, bounds the tile, so they trade operand stages for C slots.
 // FP8 variant: e4m3 K-major operands scaled per 128 x 128 block; the
 // accumulator is folded into fp32 registers after every 128-deep K block
 // with the product of the two blocks' scales.
@@ -190,7 +187,7 @@ struct GemmCfg {
   static constexpr int A_BYTES = BM * BK * ELEM;
   static constexpr int B_BYTES = BN * BK * ELEM;
   static constexpr int STAGE_BYTES = NOPS * (A_BYTES + B_BYTES);
-  static constexpr int STAGES = FP8 ? 6 : PF ? (SPLIT ? 2 : 3) : (SPLIT ? 3 : (BN == 128 ? 6 : 4));
+  static constexpr int STAGES = FP8 ? 6 : PF ? (SPLIT ? 3 : 4) : (SPLIT ? 3 : (BN == 128 ? 6 : 4));
   // TMEM: two main accumulators (alternating by round), then two corrections
   // (alternating by tile)
   static constexpr int CORR_COL = 2 * BN;
@@ -198,9 +195,8 @@ struct GemmCfg {
   static_assert(TMEM_COLS <= 512, "TMEM budget");
   static constexpr int GC = BN / kEpiGroups;              // columns of one epilogue group
   static constexpr int CHUNK_BYTES = 128 * kEpiCols * 4;  // one staged 128 x 16 fp32 chunk
-  static constexpr int C_SLOTS = PF ? (SPLIT ? 4 : 6) : 2;  // per group
-  static constexpr int SIDE = PF ? 2 : 0;                   // staging buffers for side copies, per group
-  static constexpr int GROUP_BYTES = (C_SLOTS + SIDE) * CHUNK_BYTES;
+  static constexpr int C_SLOTS = PF && !SPLIT ? 6 : 2;  // per group
+  static constexpr int GROUP_BYTES = C_SLOTS * CHUNK_BYTES;
   static constexpr int EPI_BYTES = kEpiGroups * GROUP_BYTES;
   static constexpr int BAR_BYTES = 512;
   static_assert(8 * (2 * STAGES + 7 + 2 * kEpiGroups * C_SLOTS + 2 * kTileQ) + 4 * kTileQ + 8 <= BAR_BYTES,
@@ -270,12 +266,17 @@ struct EpiK {
 template <int W>
 __device__ __forceinline__ void combine(const EpiK& k, float* S, int row, const float* v, long long gi, long long gj0,
                                         bool any_masked, float* r) {
-  int lo = 0, hi = W;
-  if (any_masked) k.keep_range<W>(gi, gj0, gj0 + W, lo, hi);
+  if (any_masked) {
+    int lo, hi;
+    k.keep_range<W>(gi, gj0, gj0 + W, lo, hi);
 #pragma unroll
-  for (int j = 0; j < W; ++j) {
-    const float old = S[j * 128 + row];
-    r[j] = (j >= lo && j < hi) ? fmaf(k.beta, old, k.alpha * v[j]) : old;
+    for (int j = 0; j < W; ++j) {
+      const float old = S[j * 128 + row];
+      r[j] = (j >= lo && j < hi) ? fmaf(k.beta, old, k.alpha * v[j]) : old;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < W; ++j) r[j] = fmaf(k.beta, S[j * 128 + row], k.alpha * v[j]);
   }
 #pragma unroll
   for (int j = 0; j < W; ++j) S[j * 128 + row] = r[j];
@@ -292,7 +293,52 @@ struct StoreK : EpiK {
   __device__ __forceinline__ explicit StoreK(const GemmArgs& a)
       : EpiK(a), C(a.C), ldc(a.ldc), ld_out(a.ld_out), N(a.N), out_m(a.out_m), out_n(a.out_n), out_hi(a.out_hi),
         out_lo(a.out_lo) {}
+  // the side copies take 8-byte stores at rows that are multiples of 4
+  __device__ __forceinline__ bool side_vec() const {
+    return tri == 0 && ((reinterpret_cast<uintptr_t>(out_hi) | reinterpret_cast<uintptr_t>(out_lo)) & 7) == 0 &&
+           (ld_out & 3) == 0;
+  }
 };
+
+// Side copies of a staged 128 x 16 chunk S (fp32, column-major) at (m0, gj),
+// written by the 128 threads of a group (t) after its values are in place:
+// eight threads take 32 rows of a column, four rows each, so the copies leave
+// as 8-byte stores. From the registers that hold a row of the chunk each value
+// would be a 2-byte store of its own, 256 a thread and tile, with its address;
+// that was most of a TRSM leaf product's epilogue.
+__device__ __forceinline__ void copy_side16(const StoreK& k, const float* S, int t, int m0, int gj) {
+  const int j = t >> 3, r0 = 4 * (t & 7);
+  if (gj + j >= k.out_n) return;
+  const long long at = (long long)m0 + r0 + (long long)(gj + j) * k.ld_out;
+  __half* hi = k.out_hi + at;
+  __half* lo = k.out_lo + at;  // used only when out_lo is set
+  const bool has_lo = k.out_lo != nullptr;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int r = r0 + 32 * q;
+    const float4 x = *reinterpret_cast<const float4*>(S + j * 128 + r);
+    const __half2 a = __floats2half2_rn(x.x, x.y), b = __floats2half2_rn(x.z, x.w);
+    const float2 fa = __half22float2(a), fb = __half22float2(b);
+    const __half2 c = __floats2half2_rn((x.x - fa.x) * k.lo_scale, (x.y - fa.y) * k.lo_scale);
+    const __half2 d = __floats2half2_rn((x.z - fb.x) * k.lo_scale, (x.w - fb.y) * k.lo_scale);
+    if (m0 + r + 4 <= k.out_m) {
+      *reinterpret_cast<uint2*>(hi + 32 * q) =
+          make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+      if (has_lo)
+        *reinterpret_cast<uint2*>(lo + 32 * q) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&c), *reinterpret_cast<const uint32_t*>(&d));
+    } else {
+      const __half h[4] = {__low2half(a), __high2half(a), __low2half(b), __high2half(b)};
+      const __half l[4] = {__low2half(c), __high2half(c), __low2half(d), __high2half(d)};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (m0 + r + i < k.out_m) {
+          hi[32 * q + i] = h[i];
+          if (has_lo) lo[32 * q + i] = l[i];
+        }
+    }
+  }
+}
 
 // Fused fp16 hi[/lo] copies of W result values of one row.
 template <int W>
@@ -319,20 +365,19 @@ __device__ __forceinline__ void load_old(const StoreK& s, float* old, bool row_o
   if (row_ok) s.keep_range<W>(gi, gj0, s.N, lo, hi);
   const float* crow = s.C + gi + gj0 * s.ldc;
 #pragma unroll
-  for (int j = 0; j < W; ++j) old[j] = (j >= lo && j < hi) ? __ldg(crow + (long long)j * s.ldc) : 0.f;
+  for (int j = 0; j < W; ++j) old[j] = (j >= lo && j < hi) ? __ldcg(crow + (long long)j * s.ldc) : 0.f;
 }
 
 // Per-element path: alpha/beta update of W consecutive columns of one row,
 // with the triangle mask and bounds; old: load_old's values (read only when
-// beta != 0).
+// beta != 0); r: the new values.
 template <int W>
-__device__ __forceinline__ void epilogue_store(const StoreK& s, const float* v, const float* old, long long gi,
-                                               long long gj0) {
+__device__ __forceinline__ void epilogue_store(const StoreK& s, const float* v, const float* old, bool row_ok,
+                                               long long gi, long long gj0, float* r) {
   const long long ldc = s.ldc;
   float* crow = s.C + gi + gj0 * ldc;
-  int lo, hi;
-  s.keep_range<W>(gi, gj0, s.N, lo, hi);
-  float r[W];
+  int lo = 0, hi = 0;
+  if (row_ok) s.keep_range<W>(gi, gj0, s.N, lo, hi);
   const bool has_beta = s.beta != 0.0f;
 #pragma unroll
   for (int j = 0; j < W; ++j) {
@@ -342,30 +387,19 @@ __device__ __forceinline__ void epilogue_store(const StoreK& s, const float* v, 
 #pragma unroll
   for (int j = 0; j < W; ++j)
     if (j >= lo && j < hi) crow[(long long)j * ldc] = r[j];
-  if (s.out_hi && gi < s.out_m) store_fp16_copies<W>(s, r, gi, gj0);
-}
-
-// Side copies of one row's W values into a staged fp16 hi/lo chunk.
-template <int W>
-__device__ __forceinline__ void stage_side(const EpiK& k, __half* Hs, __half* Ls, const float* r, int row) {
-#pragma unroll
-  for (int j = 0; j < W; ++j) {
-    const __half hv = __float2half_rn(r[j]);
-    Hs[j * 128 + row] = hv;
-    Ls[j * 128 + row] = __float2half_rn((r[j] - __half2float(hv)) * k.lo_scale);
-  }
 }
 
 // Columns [16 c, 16 c + 16) of a thread's register sums: registers cannot be
-// indexed at run time, so one predicated copy per chunk position keeps a
-// single copy of the chunk code instead of one per chunk.
+// indexed at run time, so one copy per chunk position (behind a branch: the
+// asm keeps the compiler from turning all of them into predicated moves)
+// keeps a single copy of the chunk code instead of one per chunk.
 template <int N>
 __device__ __forceinline__ void pick16(const float (&acc)[N], int c, float* v) {
 #pragma unroll
   for (int q = 0; q < N / 16; ++q)
     if (c == q) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = acc[16 * q + j];
+      for (int j = 0; j < 16; ++j) asm volatile("mov.f32 %0, %1;" : "=f"(v[j]) : "f"(acc[16 * q + j]));
     }
 }
 
@@ -377,11 +411,17 @@ __device__ __forceinline__ bool tile_staged(const GemmArgs& P, bool masked) {
   return P.tma_c && !(masked && P.beta == 0.0f);
 }
 
+// Whether a tile's chunks pass through the C slots at all: also per-element
+// tiles that make side copies, which build them from the slot.
+__device__ __forceinline__ bool tile_slots(const GemmArgs& P, bool masked) {
+  return tile_staged(P, masked) || (P.out_hi && !masked);
+}
+
 // The C loader's walk (one thread): the CTA's tiles in the epilogue's chunk
 // order, the groups in turn; a group's chunk n goes to slot n % SLOTS of its
 // ring once the epilogue has given back the slot's previous chunk
-// (n - SLOTS). Chunks the epilogue does not read (beta == 0) only pass the
-// slot's barrier.
+// (n - SLOTS). Chunks that are not loaded (beta == 0, per-element tiles) only
+// pass the slot's barrier.
 template <int SLOTS, int STRIDE>
 struct CLoader {
   float* stage;  // group g's slots start at stage + g * STRIDE
@@ -394,9 +434,11 @@ struct CLoader {
       : stage(stage_), cfull(cfull_), cfree(cfree_), armed(0), armed_phase(0) {
     for (int g = 0; g < kEpiGroups; ++g) slot[g] = 0, ph[g] = 0;
   }
-  // chunks of the tile at (m0, n0) with GC columns per group; false when a wait gave up
-  __device__ __forceinline__ bool tile(const GemmArgs& P, int m0, int n0, int gc, volatile int* abort_flag) {
-    const bool need = P.beta != 0.0f;
+  // chunks of the tile at (m0, n0) with gc columns per group; false when a wait gave up
+  __device__ __forceinline__ bool tile(const GemmArgs& P, int m0, int n0, int gc, bool masked,
+                                       volatile int* abort_flag) {
+    if (!tile_slots(P, masked)) return true;
+    const bool need = P.beta != 0.0f && P.tma_c;
     for (int c0 = 0; c0 < gc; c0 += kEpiCols) {
 #pragma unroll
       for (int g = 0; g < kEpiGroups; ++g) {
@@ -438,69 +480,67 @@ struct CLoader {
 };
 
 // One epilogue group of four warps (128 threads, named barrier `bar`).
-template <int SLOTS, int SIDE>
+template <int SLOTS>
 struct EpiGroup {
-  float* slots;               // the group's ring of 128 x 16 chunks, then SIDE fp16 hi/lo chunks
+  static constexpr bool kSlots = SLOTS > 0;
+  float* slots;               // the group's ring of 128 x 16 chunks
   uint64_t *cfull, *cfree;    // per slot: chunk (or its hand-over) arrived / slot given back
   int bar, row;               // row: this thread's row of the tile
   bool issuer;
   int slot = 0;        // next ring slot
   uint32_t phase = 0;  // its barrier's phase (flips when the ring wraps)
   int prev = -1;       // slot of the previous chunk, still to be released (-1: none)
-  int nside = 0;       // side-copy chunks staged so far (selects the buffer)
 
-  // One 128 x 16 chunk at (m0, gj) staged in the next slot: the slot holds
-  // this chunk of C when beta != 0; the result is combined in place and
-  // stored from the slot. Before the issuer stores a chunk it waits until the
-  // previous chunk's store has read its slot and gives that slot back to the
-  // loader. All 128 threads call it together; false, in every thread alike,
-  // when the slot's wait gave up. The FP16 side copies alternate between
-  // SIDE staging buffers, or (SIDE == 0) are stored from registers.
-  __device__ __forceinline__ bool chunk_staged(const GemmArgs& P, const StoreK& k, const float* v, int m0, int gj,
-                                               volatile int* abort_flag) {
+  // One 128 x 16 chunk at (m0, gj) through the next slot. Staged (TMA): the
+  // slot holds this chunk of C when beta != 0; the result is combined in place
+  // and stored from the slot. Otherwise (per-element C, old: its old values)
+  // the result is stored from registers and left in the slot for the side
+  // copies. The FP16 side copies are made from the slot after the barrier
+  // that completes the chunk; the slot goes back to the loader at the next
+  // chunk's barrier, when every thread has read it and its store has, too.
+  // All 128 threads call it together; false, in every thread alike, when the
+  // slot's wait gave up.
+  __device__ __forceinline__ bool chunk_slot(const GemmArgs& P, const StoreK& k, bool staged, bool side_vec,
+                                             bool row_ok, const float* v, const float* old, int m0, int gj,
+                                             volatile int* abort_flag) {
     constexpr int W = kEpiCols;
     float* S = slots + slot * (128 * W);
     const bool got = mbar_wait(&cfull[slot], phase, abort_flag, P.err, kDevErrTimeoutEpilogue);
     const long long gi = (long long)m0 + row;
     float r[W];
-    if (k.beta != 0.0f) {
+    if (staged && k.beta != 0.0f) {
       combine<W>(k, S, row, v, gi, gj, k.chunk_masked<W>(m0, gj), r);
     } else {
+      if (staged) {
 #pragma unroll
-      for (int j = 0; j < W; ++j) {
-        r[j] = k.alpha * v[j];
-        S[j * 128 + row] = r[j];
+        for (int j = 0; j < W; ++j) r[j] = k.alpha * v[j];
+      } else {
+        epilogue_store<W>(k, v, old, row_ok, gi, gj, r);
       }
-    }
-    const bool side = SIDE > 0 && P.tma_out && gj < k.out_n && m0 < k.out_m;
-    __half* Hs = reinterpret_cast<__half*>(slots + (SLOTS + (SIDE == 2 ? (nside & 1) : 0)) * (128 * W));
-    if constexpr (SIDE > 0) {
-      if (side) {
-        // two buffers: the store that used this one was read before the
-        // previous chunk's store was issued, which this thread has seen at the
-        // previous chunk's barrier
-        stage_side<W>(k, Hs, Hs + 128 * W, r, row);
-        ++nside;
-      }
+#pragma unroll
+      for (int j = 0; j < W; ++j) S[j * 128 + row] = r[j];
     }
     fence_proxy_async_smem();
     if (named_bar_any(bar, 128, !got)) return false;
     if (issuer) {
-      bulk_wait_read<0>();  // the previous chunk's stores have read their slot and side buffer
+      bulk_wait_read<0>();  // the previous chunk's store has read its slot, and every thread is past it
       if (prev >= 0) mbar_arrive(&cfree[prev]);
-      tma_store_2d(&P.mapC, S, m0, gj);
-      if (side) {
-        tma_store_2d(&P.mapOut[0], Hs, m0, gj);
-        if (k.out_lo) tma_store_2d(&P.mapOut[1], Hs + 128 * W, m0, gj);
+      if (staged) {
+        tma_store_2d(&P.mapC, S, m0, gj);
+        bulk_commit();
       }
-      bulk_commit();
     }
     prev = slot;
     if (++slot == SLOTS) {
       slot = 0;
       phase ^= 1u;
     }
-    if (k.out_hi && !(SIDE > 0 && P.tma_out) && gi < k.out_m) store_fp16_copies<W>(k, r, gi, gj);
+    if (k.out_hi && m0 < k.out_m && gj < k.out_n) {
+      if (side_vec)
+        copy_side16(k, S, threadIdx.x & 127, m0, gj);
+      else if (gi < k.out_m)
+        store_fp16_copies<W>(k, r, gi, gj);
+    }
     return true;
   }
 };
@@ -511,12 +551,16 @@ struct EpiGroup {
 // group's GC. (m0, gy): the group's first row and column of C. False when
 // the epilogue has to stop.
 template <int GC, class Group, class Acc>
-__device__ __forceinline__ bool epilogue_tile(const GemmArgs& P, Group& g, Acc& acc, int m0, int gy, bool staged,
+__device__ __forceinline__ bool epilogue_tile(const GemmArgs& P, Group& g, Acc& acc, int m0, int gy, bool masked,
                                               volatile int* abort_flag) {
   const StoreK sk(P);
   const long long gi = (long long)m0 + g.row;
   const bool row_ok = gi < P.M;
   const int nval = min(max((sk.N - gy + kEpiCols - 1) / kEpiCols, 0), GC / kEpiCols);  // chunks inside C
+  const bool side_vec = sk.side_vec();
+  // kSlots false: no ring (launches that read no C and make no side copies)
+  const bool staged = Group::kSlots && m0 < P.M && tile_staged(P, masked);
+  const bool through = Group::kSlots && m0 < P.M && tile_slots(P, masked);
   // per-element path: C's old values are loaded one chunk ahead, the first
   // before the accumulator wait (where the fold leaves registers for it)
   float old[kEpiCols];
@@ -530,10 +574,14 @@ __device__ __forceinline__ bool epilogue_tile(const GemmArgs& P, Group& g, Acc& 
     acc.chunk(c, v);
     if (c >= nval) continue;
     const int gj = gy + c * kEpiCols;
-    if (staged) {
-      if (!g.chunk_staged(P, sk, v, m0, gj, abort_flag)) return false;
+    if (through) {
+      if (!g.chunk_slot(P, sk, staged, side_vec, row_ok, v, old, m0, gj, abort_flag)) return false;
     } else {
-      if (row_ok) epilogue_store<kEpiCols>(sk, v, old, gi, gj);
+      float r[kEpiCols];
+      epilogue_store<kEpiCols>(sk, v, old, row_ok, gi, gj, r);
+      if (sk.out_hi && row_ok && gi < sk.out_m) store_fp16_copies<kEpiCols>(sk, r, gi, gj);
+    }
+    if (!staged) {
       if (read_old && c + 1 < nval) load_old<kEpiCols>(sk, old, row_ok, gi, gj + kEpiCols);
     }
   }
@@ -608,26 +656,20 @@ struct TileAcc {
           const float s = sc.next(kb, tile.w);
           if (!round()) return false;
           const uint32_t ta = tmem + (uint32_t)(buf * Cfg::BN);
-#pragma unroll
-          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
-            float v[32];
-            tmem_ld32(ta + c0, v);
+          tmem_for32<Cfg::GC>(ta, [&](int c0, const float* v) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(s, v[j], acc[c0 + j]);
-          }
+          });
           release(&tempty[buf]);
         }
       } else {
         for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk) {
           if (!round()) return false;
           const uint32_t ta = tmem + (uint32_t)(buf * Cfg::BN);
-#pragma unroll
-          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
-            float v[32];
-            tmem_ld32(ta + c0, v);
+          tmem_for32<Cfg::GC>(ta, [&](int c0, const float* v) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
-          }
+          });
           release(&tempty[buf]);
         }
         if (tile.z < tile.w) {  // the last round's commit covers the correction's MMAs
@@ -906,8 +948,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
            t = next_tile<false>(args, t, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutProducer)) {
         const int4 tile = args.tiles[t];
         const GemmArgs& P = tile_problem<GROUPED>(args, t);
-        if (tile_staged(P, tile_reaches_mask(P, tile.x, tile.y, BM, BN)))
-          ok = ld.tile(P, tile.x, tile.y, Cfg::GC, abort_flag);
+        ok = ld.tile(P, tile.x, tile.y, Cfg::GC, tile_reaches_mask(P, tile.x, tile.y, BM, BN), abort_flag);
       }
       ld.drain(args.err);
     }
@@ -917,7 +958,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
     const int quarter = warp & 3;  // TMEM lane quarter this warp may access
     const int group = (warp - kEpiWarp0) >> 2, gc0 = group * Cfg::GC;
     const uint32_t tmem = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)gc0;
-    EpiGroup<Cfg::C_SLOTS, Cfg::SIDE> g{stage_c + group * (Cfg::GROUP_BYTES / 4), cfull + group * Cfg::C_SLOTS,
+    EpiGroup<Cfg::C_SLOTS> g{stage_c + group * (Cfg::GROUP_BYTES / 4), cfull + group * Cfg::C_SLOTS,
                              cfree + group * Cfg::C_SLOTS, 1 + group, quarter * 32 + lane,
                              quarter == 0 && lane == 0};
     int it = 0, nt = 0;
@@ -930,8 +971,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
       const int4 tile = args.tiles[t];
       const GemmArgs& P = tile_problem<GROUPED>(args, t);
       TileAcc<Cfg> acc{args, P, tile, gc0, tmem, tfull, tempty, xempty, it, nt, abort_flag};
-      const bool staged = tile_staged(P, tile_reaches_mask(P, tile.x, tile.y, BM, BN));
-      if (!epilogue_tile<Cfg::GC>(P, g, acc, tile.x, tile.y + gc0, staged, abort_flag)) break;
+      if (!epilogue_tile<Cfg::GC>(P, g, acc, tile.x, tile.y + gc0, tile_reaches_mask(P, tile.x, tile.y, BM, BN),
+                                  abort_flag))
+        break;
     }
     if (g.issuer) bulk_wait<0>();  // all TMA stores complete before the CTA retires
   }
@@ -1000,8 +1042,8 @@ struct PairCfg {
   static constexpr int TMEM_COLS = 512;
   static constexpr int GC = BN / kEpiGroups;
   static constexpr int CHUNK_BYTES = 128 * kEpiCols * 4;
-  static constexpr int C_SLOTS = DIRECT ? 0 : (FOLD ? 2 : 4), SIDE = 0;  // per group
-  static constexpr int GROUP_BYTES = (C_SLOTS + SIDE) * CHUNK_BYTES;
+  static constexpr int C_SLOTS = DIRECT ? 0 : (FOLD ? 2 : 4);  // per group
+  static constexpr int GROUP_BYTES = C_SLOTS * CHUNK_BYTES;
   static constexpr int EPI_BYTES = kEpiGroups * GROUP_BYTES;
   static constexpr int BAR_BYTES = 320;
   static_assert(8 * (2 * STAGES + 5 + 2 * kEpiGroups * C_SLOTS) + 8 <= BAR_BYTES, "barrier space");
@@ -1063,25 +1105,19 @@ struct PairAcc {
           const int b = it & 1;
           if (!wait(b, (uint32_t)(it >> 1) & 1u)) return false;
           const uint32_t ta = tmem + (uint32_t)(b * Cfg::BN);
-#pragma unroll
-          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
-            float v[32];
-            tmem_ld32(ta + c0, v);
+          tmem_for32<Cfg::GC>(ta, [&](int c0, const float* v) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(s, v[j], acc[c0 + j]);
-          }
+          });
           release(b);
         }
       } else {
         for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk, ++it) {
           if (!wait(0, (uint32_t)it & 1u)) return false;
-#pragma unroll
-          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
-            float v[32];
-            tmem_ld32(tmem + c0, v);
+          tmem_for32<Cfg::GC>(tmem, [&](int c0, const float* v) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
-          }
+          });
           release(0);
         }
         if (tile.z < tile.w) {
@@ -1320,8 +1356,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
           for (int t = static_first(args, pair); t >= 0 && ok; t = static_next(args, pair, npairs, t)) {
             const int4 tile = args.tiles[t];
             const int m0 = tile.x + 128 * (int)rank;
-            if (m0 < args.M && tile_staged(args, tile_reaches_mask(args, m0, tile.y, 128, BN)))
-              ok = ld.tile(args, m0, tile.y, Cfg::GC, abort_flag);
+            if (m0 < args.M)  // rows wholly outside C are stored by no one
+              ok = ld.tile(args, m0, tile.y, Cfg::GC, tile_reaches_mask(args, m0, tile.y, 128, BN), abort_flag);
           }
           ld.drain(args.err);
         }
@@ -1334,7 +1370,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     const int quarter = warp & 3;
     const int group = (warp - kEpiWarp0) >> 2, gc0 = group * Cfg::GC;
     const uint32_t tmem = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)gc0;
-    EpiGroup<Cfg::C_SLOTS, Cfg::SIDE> g{stage_c + group * (Cfg::GROUP_BYTES / 4), cfull + group * Cfg::C_SLOTS,
+    EpiGroup<Cfg::C_SLOTS> g{stage_c + group * (Cfg::GROUP_BYTES / 4), cfull + group * Cfg::C_SLOTS,
                              cfree + group * Cfg::C_SLOTS, 1 + group, quarter * 32 + lane,
                              quarter == 0 && lane == 0};
     int it = 0, nt = 0;
@@ -1342,10 +1378,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       const int4 tile = args.tiles[t];
       const int m0 = tile.x + 128 * (int)rank;
       PairAcc<Cfg> acc{args, tile, m0, gc0, tmem, tfull, tempty_leader, it, nt, abort_flag};
-      // rows wholly outside C are stored by neither path
-      const bool staged = !Cfg::DIRECT && m0 < args.M &&
-                          tile_staged(args, tile_reaches_mask(args, m0, tile.y, 128, BN));
-      if (!epilogue_tile<Cfg::GC>(args, g, acc, m0, tile.y + gc0, staged, abort_flag)) break;
+      if (!epilogue_tile<Cfg::GC>(args, g, acc, m0, tile.y + gc0, tile_reaches_mask(args, m0, tile.y, 128, BN),
+                                  abort_flag))
+        break;
     }
     if (g.issuer) bulk_wait<0>();
   }

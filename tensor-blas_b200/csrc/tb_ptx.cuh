@@ -370,6 +370,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// N columns (a multiple of 32) from taddr on, handed to f(column offset, 32 values).
+template <int N, class F>
+__device__ __forceinline__ void tmem_for32(uint32_t taddr, F&& f) {
+#pragma unroll
+  for (int c = 0; c < N; c += 32) {
+    float v[32];
+    tmem_ld32(taddr + c, v);
+    f(c, v);
+  }
+}
+
 // 32 lanes x 32 columns of fp32 to TMEM; tmem_st_wait completes this thread's stores.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
   asm volatile(
