@@ -123,7 +123,7 @@ struct tb_batch_s {
   int ndiag = 0;
   long long diag_blocks = 0;
   tb::ChainJob* d_chain = nullptr;
-  int nchain = 0;
+  std::vector<int> level_jobs;  // leaves that reach each doubling level (chain is sorted by size)
   tb::GemmArgs* d_problems = nullptr;
   int* d_sched = nullptr;  // one tile counter per grouped GEMM launch
   std::vector<tb::Launch> launches;
@@ -363,7 +363,8 @@ extern "C" tb_status tb_batch_create(tb_batch_t* out, int count, const int* kind
     double* D = reinterpret_cast<double*>(base + o.d);
     if (p.leaf_start.size() > 1) add_conv(p.A, p.n, p.n, p.lda, p.ah, p.al, p.lda_h, 2);
     add_conv(p.B, p.n, std::min<long>(p.leaf, p.n), p.ldb, p.rh, p.rl, p.ldr, 0);  // first leaf's R
-    diag.push_back(DiagJob{p.A, (long long)p.lda, (long long)p.n, D, diag_blocks});
+    diag.push_back(DiagJob{p.A, (long long)p.lda, (long long)p.n, D, diag_blocks, p.wh, p.wl, p.ldw, p.wstride,
+                           (int)p.leaf});
     diag_blocks += (p.n + 31) / 32;
     for (size_t l = 0; l < p.leaf_start.size(); ++l) {
       const long s = p.leaf_start[l];
@@ -429,6 +430,13 @@ extern "C" tb_status tb_batch_create(tb_batch_t* out, int count, const int* kind
       b->launches.push_back(std::move(L));
     }
   }
+  // largest leaves first, so that a level's launch covers the jobs it needs
+  std::stable_sort(chain.begin(), chain.end(), [](const ChainJob& x, const ChainJob& y) { return x.size > y.size; });
+  for (int h = 1; h < 512 / 32; h *= 2) {
+    int jobs = 0;
+    for (const ChainJob& j : chain) jobs += (j.size + 31) / 32 > h ? 1 : 0;
+    b->level_jobs.push_back(jobs);
+  }
   Arena tab;
   const size_t o_probs = tab.take(sizeof(GemmArgs) * std::max(nprob, 1));
   const size_t o_conv = tab.take(sizeof(ConvJob) * std::max<size_t>(conv.size(), 1));
@@ -480,7 +488,6 @@ extern "C" tb_status tb_batch_create(tb_batch_t* out, int count, const int* kind
   b->ndiag = (int)diag.size();
   b->diag_blocks = diag_blocks;
   b->d_chain = reinterpret_cast<ChainJob*>(tb_ + o_chain);
-  b->nchain = (int)chain.size();
   // one-time set-up that must not happen inside a stream capture
   device_error_word();
   sm_count();
@@ -500,7 +507,7 @@ extern "C" tb_status tb_batch_run(tb_batch_t b) {
     TB_CUDA_TRY(cudaGetLastError());
     note_launch();
   }
-  TB_TRY(trsm_inverses_grouped(b->d_diag, b->ndiag, b->diag_blocks, b->d_chain, b->nchain, st));
+  TB_TRY(trsm_inverses_grouped(b->d_diag, b->ndiag, b->diag_blocks, b->d_chain, b->level_jobs, st));
   // the launches' tile counters start at zero on every run (a memset node
   // when the run is captured in a graph)
   if (!b->launches.empty()) TB_CUDA_TRY(cudaMemsetAsync(b->d_sched, 0, sizeof(int) * b->launches.size(), st));

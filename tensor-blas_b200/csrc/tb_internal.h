@@ -207,6 +207,11 @@ struct DiagJob {
   long long n;
   double* D;
   long long first;
+  // the instance's leaf inverses as FP16 hi/lo (the diagonal sub-blocks are written here)
+  __half* hi;
+  __half* lo;
+  long long ldw, wstride;
+  int leaf;
 };
 // One leaf inverse (rows/cols [s, s+size) of A) as FP16 hi/lo, column-major.
 struct ChainJob {
@@ -217,16 +222,15 @@ struct ChainJob {
   __half* Whi;
   __half* Wlo;
   long long ldw;
-  double* Wg;  // FP64 working panels of the inverse (ldw x size)
+  double* Wg;  // the inverse in FP64 (ldw x size rounded up to 32)
 };
 tb_status trsm_inverses_grouped(const DiagJob* d_diag, int ndiag, long long nblocks, const ChainJob* d_chain,
-                                int nchain, cudaStream_t st);
-// FP64 inverses of the diagonal leaf blocks {s, size} (s a multiple of 32,
-// size <= 512) of an FP64 lower-triangular matrix of order nt; W_b at
+                                const std::vector<int>& level_jobs, cudaStream_t st);
+// FP64 inverses of the diagonal leaf blocks (`leaf` rows each, a multiple of
+// 32, <= 512) of an FP64 lower-triangular matrix of order nt; W_b at
 // W + b * wstride, leading dimension ldw. D: (nt + 31) / 32 * 1024 doubles.
-tb_status trsm_leaf_inverses_f64(long nt, const double* A, long lda, const int2* d_leaves, int nleaf, int max_size,
-                                 double* D, double* W, long long ldw, long long wstride, cudaStream_t st,
-                                 bool unit = false);
+tb_status trsm_leaf_inverses_f64(long nt, const double* A, long lda, int leaf, int nleaf, double* D, double* W,
+                                 long long ldw, long long wstride, cudaStream_t st, bool unit = false);
 // FP32 TRSM with its triangular operand prepared once (FP16 copy, leaf
 // inverses) and applied to one or more right-hand-side blocks.
 struct TrsmCtx {
@@ -273,10 +277,6 @@ struct PrepConv {  // fp32 rows x cols (lds) -> fp16 hi [lo] (ldd), triangle mod
 struct PrepJobs {
   PrepConv conv[2];
   int nconv = 0;
-  const float* A = nullptr;  // 32 x 32 FP64 inverses of A's diagonal (order n) into D
-  long long lda = 0, n = 0;
-  double* D = nullptr;
-  bool unit = false;
   int* zero = nullptr;  // nzero ints set to 0
   long long nzero = 0;
 };

@@ -1576,9 +1576,7 @@ tb_status ozaki_trsm_impl(bool right, long m, long n, const double* A, long lda,
   long leaf = round_up(std::min<long>(nb, kOzLeaf), 64);
   if (leaf > kOzLeaf) leaf = kOzLeaf;
   c.leaf = (int)leaf;
-  std::vector<int2> leaves;
-  for (long s = 0; s < nt; s += leaf) leaves.push_back(make_int2((int)s, (int)std::min<long>(leaf, nt - s)));
-  const long nleaf = (long)leaves.size();
+  const long nleaf = (nt + leaf - 1) / leaf;
   c.ldw = leaf;
   c.wstride = leaf * leaf;
   const long other = right ? m : n;  // extent of B across the solve
@@ -1586,18 +1584,15 @@ tb_status ozaki_trsm_impl(bool right, long m, long n, const double* A, long lda,
   const size_t g_bytes = oz_gemm_ws(std::max<long>(other, nt), std::max<long>(other, nt), nt / 2 + leaf, S);
   const size_t w_bytes = (size_t)round_up((long long)c.wstride * nleaf * 8, 256);
   const size_t d_bytes = (size_t)round_up((nt + 31) / 32 * 1024 * 8, 256);
-  const size_t l_bytes = (size_t)round_up(nleaf * (long long)sizeof(int2), 256);
-  char* ws = static_cast<char*>(pool_get(w_bytes + d_bytes + l_bytes + g_bytes));
+  char* ws = static_cast<char*>(pool_get(w_bytes + d_bytes + g_bytes));
   if (!ws) {
-    set_last_error("ozaki trsm: cannot allocate %zu bytes of scratch", w_bytes + d_bytes + l_bytes + g_bytes);
+    set_last_error("ozaki trsm: cannot allocate %zu bytes of scratch", w_bytes + d_bytes + g_bytes);
     return TB_ERROR_ALLOC;
   }
   c.W = reinterpret_cast<double*>(ws);
   double* D = reinterpret_cast<double*>(ws + w_bytes);
-  int2* dleaves = reinterpret_cast<int2*>(ws + w_bytes + d_bytes);
-  c.ws = ws + w_bytes + d_bytes + l_bytes;
-  TB_CUDA_TRY(cudaMemcpyAsync(dleaves, leaves.data(), nleaf * sizeof(int2), cudaMemcpyHostToDevice, st));
-  TB_TRY(trsm_leaf_inverses_f64(nt, A, lda, dleaves, (int)nleaf, (int)leaf, D, c.W, c.ldw, c.wstride, st));
+  c.ws = ws + w_bytes + d_bytes;
+  TB_TRY(trsm_leaf_inverses_f64(nt, A, lda, (int)leaf, (int)nleaf, D, c.W, c.ldw, c.wstride, st));
   return oz_trsm_rec(c, 0, nt);
 }
 

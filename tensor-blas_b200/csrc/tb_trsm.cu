@@ -14,8 +14,8 @@
 //    the reference does with B1 (BLAS/tc_trsm.cu:59-66).
 //  * The leaf replaces FP32 cublasStrsm with X_b = B_b * inv(A_bb)^T (or
 //    inv(A_bb) * B_b): inv(A_bb) is computed in FP64 by warp-level
-//    substitution on 32x32 diagonal sub-blocks plus blocked 32-wide column
-//    chains in shared memory, and applied with the split-FP16 3-product
+//    substitution on 32x32 diagonal sub-blocks and doubling (pairs of
+//    inverses joined by two products per level), and applied with the split-FP16 3-product
 //    tensor-core GEMM, i.e. FP32-level accuracy like the reference's leaf.
 //  * Split points are multiples of 64 so every TMA coordinate stays aligned.
 //    For n = nb * 2^L (the configured 16384 / 512) the leaves coincide with
@@ -34,74 +34,138 @@ namespace {
 
 constexpr int kLeafMax = 512;  // largest diagonal block inverted explicitly
 
+// Where the FP16 hi/lo pairs of the leaf inverses live: leaf b's W at
+// hi + b * stride (lo likewise), leading dimension ld; leaves of `leaf` rows.
+struct WOut {
+  __half *hi, *lo;
+  long long ld, stride;
+  int leaf;
+};
+
 // Inverse of each 32x32 diagonal sub-block of A (rows/cols >= n padded with
 // the identity). One warp per sub-block; lane c owns column c of the inverse
-// and runs forward substitution in FP64 registers; rows of L are broadcast
-// from shared memory. Output: D[t*1024 + i + 32*c] (column-major 32x32).
+// and runs forward substitution in FP64: row i's quotient is subtracted from
+// all later sums at once. Output: D[t*1024 + i + 32*c] (column-major 32x32),
+// and with `out` the sub-block's place in its leaf's FP16 hi/lo pair.
+//
+// A warp runs this once, so what it costs is mostly fetching the code: fully
+// unrolled in registers (about 2500 instructions) a launch took 18 to 24 us
+// however the substitution was arranged. The loop over the rows stays rolled,
+// the columns in shared memory: 20 us.
+struct DiagSmem {
+  double L[32][33];  // L[i][j], row i
+  double w[32][32];  // w[i][c]: column c of the inverse
+};
+
 template <class T>
 __device__ __forceinline__ void diag_inv32_body(long long n, const T* __restrict__ A, long long lda,
-                                                double* __restrict__ D, long long t, bool unit, double (*L)[33],
-                                                int c) {
+                                                double* __restrict__ D, long long t, bool unit, DiagSmem& s, int c,
+                                                const WOut* out) {
   const long long base = t * 32;
-  for (int i = 0; i < 32; ++i) {
-    const long long gi = base + i, gj = base + c;
-    double v;
-    if (gi < n && gj < n)
-      v = (i > c || (i == c && !unit)) ? (double)A[gi + gj * lda] : (i == c ? 1.0 : 0.0);
-    else
-      v = (i == c) ? 1.0 : 0.0;
-    L[i][c] = v;
+#pragma unroll 8
+  for (int j = 0; j < 32; ++j) {  // lane c: row c of the sub-block, column j
+    const long long gi = base + c, gj = base + j;
+    s.L[c][j] =
+        (gi < n && gj < n && (c > j || (c == j && !unit))) ? (double)A[gi + gj * lda] : (c == j ? 1.0 : 0.0);
+    s.w[j][c] = c == j ? 1.0 : 0.0;
   }
   __syncwarp();
-  double w[32];
-#pragma unroll
+  // FP32 operands: the 32 divisors' reciprocals side by side, then quotients
+  // with one residual correction (Markstein 1990), which leaves them correctly
+  // rounded but for rare last bits; where a divisor or quotient is not finite
+  // the plain product stands. FP64 operands divide: their reciprocals may
+  // overflow.
+  constexpr bool kRecip = sizeof(T) == 4;
+  const double rc = kRecip ? 1.0 / s.L[c][c] : 0.0;
+#pragma unroll 1
   for (int i = 0; i < 32; ++i) {
-    double s = (i == c) ? 1.0 : 0.0;
+    const double x = s.w[i][c], d = s.L[i][i];
+    // the rows below, in groups of 8, are on their way before the quotient is ready
+    double l[32], w[32];
 #pragma unroll
-    for (int p = 0; p < i; ++p) s -= L[i][p] * w[p];
-    w[i] = (i < c) ? 0.0 : s / L[i][i];
+    for (int g = 0; g < 4; ++g)
+      if (8 * g + 7 > i) {
+#pragma unroll
+        for (int r = 8 * g; r < 8 * g + 8; ++r) l[r] = s.L[r][i], w[r] = s.w[r][c];
+      }
+    double q;
+    if (kRecip) {
+      const double r = __shfl_sync(0xffffffffu, rc, i);
+      q = x * r;
+      const double e = fma(-q, d, x);
+      if (fabs(e) <= 1.7976931348623157e308) q = fma(e, r, q);
+    } else {
+      q = x / d;
+    }
+    if (i < c) q = 0.0;
+    s.w[i][c] = q;
+#pragma unroll
+    for (int g = 0; g < 4; ++g)
+      if (8 * g + 7 > i) {
+#pragma unroll
+        for (int r = 8 * g; r < 8 * g + 8; ++r)
+          if (r > i) s.w[r][c] = w[r] - l[r] * q;
+      }
   }
-#pragma unroll
-  for (int i = 0; i < 32; ++i) D[t * 1024 + i + 32 * c] = w[i];
+  __syncwarp();
+#pragma unroll 8
+  for (int j = 0; j < 32; ++j) D[t * 1024 + c + 32 * j] = s.w[c][j];  // lane c: row c
+  if (!out || base + c >= n) return;
+  const long long b = base / out->leaf, l0 = base - b * out->leaf;
+  __half* h = out->hi + b * out->stride + l0 + c + l0 * out->ld;
+  __half* l = out->lo + b * out->stride + l0 + c + l0 * out->ld;
+#pragma unroll 4
+  for (int j = 0; j < 32; ++j) {
+    if (base + j >= n) break;
+    const double v = s.w[c][j];
+    const __half x = __float2half_rn((float)v);
+    h[j * out->ld] = x;
+    l[j * out->ld] = __float2half_rn((float)((v - (double)__half2float(x)) * 2048.0));
+  }
+}
+
+// One warp per sub-block, two to a block; out.hi == nullptr: D only.
+constexpr int kDiagThreads = 64;
+
+template <class T>
+__global__ void __launch_bounds__(kDiagThreads)
+    diag_inv32_kernel(long long n, const T* __restrict__ A, long long lda, double* __restrict__ D, bool unit,
+                      const WOut out) {
+  extern __shared__ __align__(16) uint8_t diag_smem[];
+  DiagSmem* s = reinterpret_cast<DiagSmem*>(diag_smem);
+  const int warp = threadIdx.x >> 5;
+  const long long t = (long long)blockIdx.x * (kDiagThreads / 32) + warp;
+  if (t * 32 < n)
+    diag_inv32_body<T>(n, A, lda, D, t, unit, s[warp], threadIdx.x & 31, out.hi ? &out : nullptr);
 }
 
 template <class T>
-__global__ void __launch_bounds__(32) diag_inv32_kernel(long long n, const T* __restrict__ A, long long lda,
-                                                        double* __restrict__ D, bool unit) {
-  __shared__ double L[32][33];
-  diag_inv32_body<T>(n, A, lda, D, blockIdx.x, unit, L, threadIdx.x);
+tb_status diag_inv32(long long n, const T* A, long long lda, double* D, bool unit, const WOut& out, cudaStream_t st) {
+  constexpr int per = kDiagThreads / 32;
+  diag_inv32_kernel<T><<<(unsigned)(((n + 31) / 32 + per - 1) / per), kDiagThreads, per * sizeof(DiagSmem), st>>>(n, A, lda, D, unit,
+                                                                                           out);
+  TB_CUDA_TRY(cudaGetLastError());
+  note_launch();
+  return TB_SUCCESS;
 }
 
-// The preparation of a TRSM in one launch: FP32 -> FP16 conversions (A's
-// lower part, and for the persistent solve the first leaf block of B), the
-// 32 x 32 FP64 inverses of A's diagonal (warps 0..3 of a block, one
-// sub-block each) and the zeroing of an int array (the persistent solve's
-// progress counters), as consecutive ranges of one 1-D grid. Each job does
-// exactly what its own kernel would (same element arithmetic).
+// The conversions of a TRSM's preparation in one launch: FP32 -> FP16 copies
+// (A's lower part and the first leaf block of B) and the zeroing of an int
+// array (the persistent solve's progress counters), as consecutive ranges of
+// one 1-D grid. Each job does exactly what its own kernel would (same element
+// arithmetic).
 struct PrepDev {
   PrepConv conv[2];
   int conv_vec[2];
   long long conv_gx[2], conv_base[2], conv_blocks[2];
   int nconv;
-  const float* A;
-  long long lda, n;
-  double* D;
-  int unit;
-  long long diag_base, diag_blocks;
   int* zero;
   long long nzero, zero_base, zero_blocks;
 };
 
 constexpr int kPrepThreads = 256;
 
-// Launches with the diagonal-inverse job get 4 x 32 x 33 doubles of dynamic
-// shared memory (the conversion-only launches none, so their blocks pack
-// densely on the SMs).
-constexpr int kPrepDiagSmem = 4 * 32 * 33 * (int)sizeof(double);
-
 __global__ void __launch_bounds__(kPrepThreads) trsm_prep_kernel(const __grid_constant__ PrepDev p) {
-  extern __shared__ double prep_smem[];
-  double(*L)[32][33] = reinterpret_cast<double(*)[32][33]>(prep_smem);
   const long long b = blockIdx.x;
   for (int z = 0; z < p.nconv; ++z)
     if (b >= p.conv_base[z] && b < p.conv_base[z] + p.conv_blocks[z]) {
@@ -116,13 +180,6 @@ __global__ void __launch_bounds__(kPrepThreads) trsm_prep_kernel(const __grid_co
                             c.tri, 0);
       return;
     }
-  if (b >= p.diag_base && b < p.diag_base + p.diag_blocks) {
-    const int warp = threadIdx.x >> 5;
-    if (warp >= 4) return;
-    const long long t = (b - p.diag_base) * 4 + warp;
-    if (t * 32 < p.n) diag_inv32_body<float>(p.n, p.A, p.lda, p.D, t, p.unit != 0, L[warp], threadIdx.x & 31);
-    return;
-  }
   if (b >= p.zero_base && b < p.zero_base + p.zero_blocks) {
     for (long long i = (b - p.zero_base) * kPrepThreads + threadIdx.x; i < p.nzero; i += p.zero_blocks * kPrepThreads)
       p.zero[i] = 0;
@@ -142,167 +199,253 @@ __global__ void __launch_bounds__(32) diag_inv32_grouped_kernel(const DiagJob* _
       hi = mid - 1;
   }
   const DiagJob& jb = jobs[lo];
-  __shared__ double L[32][33];
-  diag_inv32_body<float>(jb.n, jb.A, jb.lda, jb.D, b - jb.first, false, L, threadIdx.x);
+  __shared__ DiagSmem s;
+  const WOut out{jb.hi, jb.lo, jb.ldw, jb.wstride, jb.leaf};
+  diag_inv32_body<float>(jb.n, jb.A, jb.lda, jb.D, b - jb.first, false, s, threadIdx.x, &out);
 }
 
-// Column chain j of the inverse of leaf block b (rows/cols [s, s+size)):
-//   W[i][j] = -Dinv_i * sum_{p=j}^{i-1} L[i][p] W[p][j]   (32x32 sub-blocks)
-// The growing 32-wide column panel of W is kept in global memory (FP64,
-// column-major, leading dimension ldg); each 32x32 sub-block of L, each W
-// block and each Dinv_i is staged (transposed) through a 32 x 32 shared tile
-// with coalesced loads, and each of the 128 threads owns a 2 x 4 block of
-// the 32x32 result so every shared-memory load feeds several FMAs. A CTA
-// needs ~27 KB of shared memory, so several share an SM and all panels of
-// all leaves run concurrently. The result is written as the FP16 hi/lo pair
-// (lo scaled by 2^11) of W with leading dimension ldw, or, without hi, the
-// FP64 panel is W itself; zeros above the diagonal.
+// Leaf inverses by doubling. With the 32 x 32 diagonal blocks inverted, a
+// level of h sub-blocks joins neighbouring inverses of h sub-blocks each,
+//   W21 = -W22 * (L21 * W11),
+// in two products (T = L21 W11, then -W22 T), each a launch in which every
+// 32 x 32 tile of every pair of every leaf is one CTA (level 1, one tile per
+// pair, does both in one). The serial path of a 512 leaf is 7 launches whose
+// CTAs run at most 8 products of 32^3 each; forward substitution by column
+// panels was one launch with 120 such products in a row: 371 us for the 32
+// leaves of an order-16384 solve and 244 us for 9, against 145 us and 74 us.
+//
+// W is kept in FP64 in global memory (column-major, leading dimension ldg),
+// off-diagonal sub-blocks in place, diagonal ones in D. T takes the unused
+// mirrored place above the diagonal, transposed (T's rows along columns), so
+// that a ragged second block always fits. Each product step stages a 32 x 32
+// block of either operand through shared memory, double-buffered, the next
+// step's loads in flight during the products.
+// Results leave as FP64 W and as the FP16 hi/lo pair (lo scaled by 2^11) with
+// the mirrored sub-block zeroed; the diagonal sub-blocks' pairs come from
+// diag_inv32_body. Without hi, W itself is the result.
 constexpr int kChainThreads = 128;
 
-template <class T>
-__device__ __forceinline__ void trtri_panel_body(const T* __restrict__ A, long long lda, int s, int size,
-                                                 const double* __restrict__ D, __half* __restrict__ hi,
-                                                 __half* __restrict__ lo, double* __restrict__ Wg, long long ldg,
-                                                 long long ldw, int j) {
-  // two staging buffers: sub-block p + 1 is loaded into registers while p's
-  // products run, so each step of the chain waits on one barrier and its
-  // global loads overlap the FMAs
-  __shared__ __align__(16) double LsT[2][32][34];  // LsT[b][k][r] = L(r, k) of a staged sub-block (or Dinv_i)
-  __shared__ __align__(16) double Ts[32][36];      // Ts[k][c]
-  __shared__ __align__(16) double Wb[2][32][36];   // Wb[b][k][c] = W(32p + k, 32j + c)
-  const int nsub = (size + 31) / 32;
-  if (j >= nsub) return;
-  const int tid = threadIdx.x;
-  const int r0 = 2 * (tid & 15), c0 = 4 * (tid >> 4);  // 2 x 4 output block
-  const int lr = tid & 31, lc = tid >> 5;              // load role: row lr, columns lc + 4q
-  const long long sub0 = (long long)s / 32;
-  double* Wp = Wg + (long long)(32 * j) * ldg;  // panel column 0 = leaf column 32j
-  for (int q = 0; q < 8; ++q) {
-    const int c = lc + 4 * q;
-    Wp[32 * j + lr + c * ldg] = D[(sub0 + j) * 1024 + lr + 32 * c];
-  }
-  __syncthreads();
-  for (int i = j + 1; i < nsub; ++i) {
-    double acc[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-    double ra[8], rw[8];
-    auto fetch = [&](int p) {
+struct LeafRef {
+  const void* A;  // rows/cols from the leaf's start
+  long long lda;
+  int size;
+  const double* D;  // the leaf's first 32 x 32 inverse
+  double* W;
+  long long ldg;
+  __half *hi, *lo;
+  long long ldw;
+};
+
+struct InvSmem {
+  double LsT[2][32][36];  // LsT[b][k][r]: left operand (r, k)
+  double Rs[2][32][36];   // Rs[b][k][c]: right operand (k, c)
+};
+
+// acc += the product of left sub-block (r, k) and right sub-block (k, c) on
+// the FP64 tensor cores (m8n8k4): warp w owns rows 16 (w & 1) .. + 15 and
+// columns 16 (w >> 1) .. + 15 as 2 x 2 tiles; a lane's pair of tile (a, b) is
+// row 8a + lane / 4, columns 8b + 2 (lane % 4) and the next. Per-thread 2 x 4
+// blocks of plain FMAs loaded three 16-byte words per 8 FMAs and were bound by
+// shared memory at a quarter of the FP64 rate.
+__device__ __forceinline__ void inv_mma(const InvSmem& s, int buf, int wr, int wc, double (&acc)[2][2][2]) {
+  const int lane = threadIdx.x & 31, kq = lane & 3, rq = lane >> 2;
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int cc = lc + 4 * q;
-        const int gr = 32 * i + lr, gc = 32 * p + cc;
-        ra[q] = (gr < size && gc < size) ? (double)A[(long long)s + gr + ((long long)s + gc) * lda] : 0.0;
-        rw[q] = __ldcg(Wp + 32 * p + lr + (long long)cc * ldg);
-      }
-    };
-    fetch(j);
-    int bsel = 0;
-    for (int p = j; p < i; ++p) {
-      bsel = (p - j) & 1;
-      // buffer bsel was last read in step p - 2, which every thread finished
-      // before the barrier of step p - 1
+  for (int k = 0; k < 32; k += 4) {
+    double a[2], b[2];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int cc = lc + 4 * q;
-        LsT[bsel][cc][lr] = ra[q];
-        Wb[bsel][lr][cc] = rw[q];
-      }
-      __syncthreads();
-      if (p + 1 < i) fetch(p + 1);
-#pragma unroll 4
-      for (int kk = 0; kk < 32; ++kk) {
-        const double2 l = *reinterpret_cast<const double2*>(&LsT[bsel][kk][r0]);
-        const double2 w01 = *reinterpret_cast<const double2*>(&Wb[bsel][kk][c0]);
-        const double2 w23 = *reinterpret_cast<const double2*>(&Wb[bsel][kk][c0 + 2]);
-        acc[0][0] = fma(l.x, w01.x, acc[0][0]);
-        acc[0][1] = fma(l.x, w01.y, acc[0][1]);
-        acc[0][2] = fma(l.x, w23.x, acc[0][2]);
-        acc[0][3] = fma(l.x, w23.y, acc[0][3]);
-        acc[1][0] = fma(l.y, w01.x, acc[1][0]);
-        acc[1][1] = fma(l.y, w01.y, acc[1][1]);
-        acc[1][2] = fma(l.y, w23.x, acc[1][2]);
-        acc[1][3] = fma(l.y, w23.y, acc[1][3]);
-      }
+    for (int i = 0; i < 2; ++i) {
+      a[i] = s.LsT[buf][k + kq][wr + 8 * i + rq];
+      b[i] = s.Rs[buf][k + kq][wc + 8 * i + rq];
     }
-    // Ts was last read by the previous step's tail, behind its final barrier;
-    // Dinv_i goes into the staging buffer the last product step did not read
-    const int dsel = bsel ^ 1;
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int b = 0; b < 4; ++b) Ts[r0 + a][c0 + b] = acc[a][b];
+      for (int j = 0; j < 2; ++j)
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                     : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+                     : "d"(a[i]), "d"(b[j]));
+  }
+}
+
+// One 32 x 32 tile of level h: PHASE 0 writes T, 1 writes W21, 2 (h == 1)
+// does both. x: the tile's index among the leaf's pairs, h * h each.
+template <class T, int PHASE>
+__device__ __forceinline__ void inv_tile(const LeafRef& f, int h, int x) {
+  __shared__ __align__(16) InvSmem s;
+  const int nsub = (f.size + 31) / 32;
+  const int pair = x / (h * h), i = (x / h) % h, j = x % h;
+  const int gi = 2 * pair * h + h + i, gj = 2 * pair * h + j;  // sub-block row and column of W21
+  if (gi >= nsub) return;
+  const int tid = threadIdx.x;
+  const int lr = tid & 31, lc = tid >> 5;                     // load role: row lr, columns lc + 4q
+  const int wr = 16 * (lc & 1), wc = 16 * (lc >> 1);          // the warp's quadrant
+  const int r0 = wr + (lr >> 2), c0 = wc + 2 * (lr & 3);      // this lane's row and column in tile (0, 0)
+  const T* A = static_cast<const T*>(f.A);
+  double acc[2][2][2] = {};
+  double ra[8], rb[8];
+  // L(gi, gk) with rows/columns beyond the leaf read as zero
+  auto load_l = [&](int gk, double* v) {
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const int cc = lc + 4 * q;
-      LsT[dsel][cc][lr] = D[(sub0 + i) * 1024 + lr + 32 * cc];
+      const int gr = 32 * gi + lr, gc = 32 * gk + lc + 4 * q;
+      v[q] = (gr < f.size && gc < f.size) ? (double)A[gr + (long long)gc * f.lda] : 0.0;
+    }
+  };
+  // W(a, b), a >= b
+  auto load_w = [&](int a, int b, double* v) {
+    const double* p = a == b ? f.D + a * 1024 : f.W + 32 * a + 32ll * b * f.ldg;
+    const long long ld = a == b ? 32 : f.ldg;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = __ldcg(p + lr + (long long)(lc + 4 * q) * ld);
+  };
+  // T(gk, gj), stored transposed in the mirrored place
+  auto load_t = [&](int gk, double* v) {
+    const double* p = f.W + 32 * gj + 32ll * gk * f.ldg;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = __ldcg(p + lr + (long long)(lc + 4 * q) * f.ldg);
+  };
+  // left blocks by columns (row lr, k = lc + 4q); right ones by columns of W
+  // (k = lr, c = lc + 4q) or of the transposed T (c = lr, k = lc + 4q)
+  auto stage = [&](int b, bool right_t) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      s.LsT[b][lc + 4 * q][lr] = ra[q];
+      if (right_t)
+        s.Rs[b][lc + 4 * q][lr] = rb[q];
+      else
+        s.Rs[b][lr][lc + 4 * q] = rb[q];
+    }
+  };
+  const int k0 = PHASE == 1 ? 2 * pair * h + h : gj, k1 = PHASE == 1 ? gi + 1 : 2 * pair * h + h;
+  auto fetch = [&](int gk) {
+    if (PHASE == 1) {
+      load_w(gi, gk, ra);
+      load_t(gk, rb);
+    } else {
+      load_l(gk, ra);
+      load_w(gk, gj, rb);
+    }
+  };
+  fetch(k0);
+  for (int gk = k0; gk < k1; ++gk) {
+    const int b = (gk - k0) & 1;
+    // buffer b was last read two steps ago, which every thread finished
+    // before the barrier of the step in between
+    stage(b, PHASE == 1);
+    __syncthreads();
+    if (gk + 1 < k1) fetch(gk + 1);
+    inv_mma(s, b, wr, wc, acc);
+  }
+  if (PHASE == 2) {  // h == 1: the second product with this tile's own T
+    load_w(gi, gi, ra);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s.LsT[1][lc + 4 * q][lr] = ra[q];
+#pragma unroll
+    for (int x2 = 0; x2 < 8; ++x2) {
+      const int a = x2 >> 2, b = (x2 >> 1) & 1, e = x2 & 1;
+      s.Rs[1][r0 + 8 * a][c0 + 8 * b + e] = acc[a][b][e];
+      acc[a][b][e] = 0.0;
     }
     __syncthreads();
-    double o[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
-#pragma unroll 4
-    for (int kk = 0; kk < 32; ++kk) {
-      const double2 d = *reinterpret_cast<const double2*>(&LsT[dsel][kk][r0]);
-      const double2 t01 = *reinterpret_cast<const double2*>(&Ts[kk][c0]);
-      const double2 t23 = *reinterpret_cast<const double2*>(&Ts[kk][c0 + 2]);
-      o[0][0] = fma(-d.x, t01.x, o[0][0]);
-      o[0][1] = fma(-d.x, t01.y, o[0][1]);
-      o[0][2] = fma(-d.x, t23.x, o[0][2]);
-      o[0][3] = fma(-d.x, t23.y, o[0][3]);
-      o[1][0] = fma(-d.y, t01.x, o[1][0]);
-      o[1][1] = fma(-d.y, t01.y, o[1][1]);
-      o[1][2] = fma(-d.y, t23.x, o[1][2]);
-      o[1][3] = fma(-d.y, t23.y, o[1][3]);
-    }
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) Wp[32 * i + r0 + a + (long long)(c0 + b) * ldg] = o[a][b];
-    __syncthreads();  // the new W block is visible to the CTA before it is staged
+    inv_mma(s, 1, wr, wc, acc);
   }
-  // columns [32j, 32j+32) of W for all rows of the leaf (zeros above the diagonal)
-  for (int q = 0; q < 8; ++q) {
-    const int c = lc + 4 * q;
-    const int gc = 32 * j + c;
-    if (gc >= size) continue;
-    for (int row = lr; row < size; row += 32) {
-      if (!hi) {
-        if (row < 32 * j) Wp[row + (long long)c * ldg] = 0.0;  // FP64 output: the panel is W itself
-        continue;
+  if constexpr (PHASE == 0) {
+#pragma unroll
+    for (int x2 = 0; x2 < 8; ++x2) {
+      const int a = x2 >> 2, b = (x2 >> 1) & 1, e = x2 & 1;
+      f.W[32 * gj + c0 + 8 * b + e + (32ll * gi + r0 + 8 * a) * f.ldg] = acc[a][b][e];
+    }
+  } else {
+#pragma unroll
+    for (int x2 = 0; x2 < 8; ++x2) {
+      const int a = x2 >> 2, b = (x2 >> 1) & 1, e = x2 & 1;
+      const int gr = 32 * gi + r0 + 8 * a, gc = 32 * gj + c0 + 8 * b + e;
+      const double v = -acc[a][b][e];
+      f.W[gr + (long long)gc * f.ldg] = v;
+      if (!f.hi || gr >= f.size) continue;  // gc < gr
+      const __half h16 = __float2half_rn((float)v);
+      f.hi[gr + (long long)gc * f.ldw] = h16;
+      f.lo[gr + (long long)gc * f.ldw] = __float2half_rn((float)((v - (double)__half2float(h16)) * 2048.0));
+    }
+    if (f.hi) {  // the mirrored sub-block of the pair: zeros
+      for (int q = 0; q < 8; ++q) {
+        const int gr = 32 * gj + lr, gc = 32 * gi + lc + 4 * q;
+        if (gc >= f.size) break;
+        f.hi[gr + (long long)gc * f.ldw] = __float2half_rn(0.f);
+        f.lo[gr + (long long)gc * f.ldw] = __float2half_rn(0.f);
       }
-      const double v = row >= 32 * j ? __ldcg(Wp + row + (long long)c * ldg) : 0.0;
-      const __half h = __float2half_rn((float)v);
-      hi[row + (long long)gc * ldw] = h;
-      lo[row + (long long)gc * ldw] = __float2half_rn((float)((v - (double)__half2float(h)) * 2048.0));
     }
   }
 }
 
-__global__ void __launch_bounds__(kChainThreads) trtri_chain_kernel(const float* __restrict__ A, long long lda,
-                                                                    const int2* __restrict__ leaves,
-                                                                    const double* __restrict__ D,
-                                                                    __half* __restrict__ Whi, __half* __restrict__ Wlo,
-                                                                    long long ldw, long long wstride,
-                                                                    double* __restrict__ Wg) {
-  const int2 leaf = leaves[blockIdx.y];  // {s, size}
-  trtri_panel_body<float>(A, lda, leaf.x, leaf.y, D, Whi + (long long)blockIdx.y * wstride,
-                          Wlo + (long long)blockIdx.y * wstride, Wg + (long long)blockIdx.y * wstride, ldw, ldw,
-                          blockIdx.x);
+// Leaves [b * leaf, (b + 1) * leaf) of one matrix of order n along blockIdx.y.
+template <class T, int PHASE>
+__global__ void __launch_bounds__(kChainThreads)
+    trtri_level_kernel(const T* __restrict__ A, long long lda, long long n, int leaf, const double* __restrict__ D,
+                       double* W, long long ldg, __half* hi, __half* lo, long long ldw, long long wstride, int h) {
+  const long long b = blockIdx.y, s = b * leaf;
+  LeafRef f;
+  f.A = A + s + s * lda;
+  f.lda = lda;
+  f.size = (int)min((long long)leaf, n - s);
+  f.D = D + s / 32 * 1024;
+  f.W = W + b * wstride;
+  f.ldg = ldg;
+  f.hi = hi ? hi + b * wstride : nullptr;
+  f.lo = lo ? lo + b * wstride : nullptr;
+  f.ldw = ldw;
+  inv_tile<T, PHASE>(f, h, blockIdx.x);
 }
 
-// FP64 operand, FP64 inverse (the Ozaki-scheme FP64 TRSM's leaves); the
-// output W itself holds the panels.
-__global__ void __launch_bounds__(kChainThreads) trtri_chain_f64_kernel(const double* __restrict__ A, long long lda,
-                                                                        const int2* __restrict__ leaves,
-                                                                        const double* __restrict__ D,
-                                                                        double* __restrict__ W, long long ldw,
-                                                                        long long wstride) {
-  const int2 leaf = leaves[blockIdx.y];
-  trtri_panel_body<double>(A, lda, leaf.x, leaf.y, D, nullptr, nullptr, W + (long long)blockIdx.y * wstride, ldw, ldw,
-                           blockIdx.x);
-}
-
-// Grouped form: one job per (instance, leaf) along blockIdx.y.
-__global__ void __launch_bounds__(kChainThreads) trtri_chain_grouped_kernel(const ChainJob* __restrict__ jobs) {
+// Grouped form: one job per (instance, leaf) along blockIdx.y, largest first.
+template <int PHASE>
+__global__ void __launch_bounds__(kChainThreads) trtri_level_grouped_kernel(const ChainJob* __restrict__ jobs, int h) {
   const ChainJob& jb = jobs[blockIdx.y];
-  trtri_panel_body<float>(jb.A, jb.lda, jb.s, jb.size, jb.D, jb.Whi, jb.Wlo, jb.Wg, jb.ldw, jb.ldw, blockIdx.x);
+  LeafRef f;
+  f.A = jb.A + jb.s + (long long)jb.s * jb.lda;
+  f.lda = jb.lda;
+  f.size = jb.size;
+  f.D = jb.D + jb.s / 32 * 1024;
+  f.W = jb.Wg;
+  f.ldg = jb.ldw;
+  f.hi = jb.Whi;
+  f.lo = jb.Wlo;
+  f.ldw = jb.ldw;
+  inv_tile<float, PHASE>(f, h, blockIdx.x);
+}
+
+// FP64 results (no FP16 pair): the diagonal sub-blocks from D, zeros above
+// the diagonal (where T was kept).
+__global__ void __launch_bounds__(256) trtri_finish_f64_kernel(long long n, int leaf, const double* __restrict__ D,
+                                                               double* __restrict__ W, long long ldw,
+                                                               long long wstride) {
+  const long long b = blockIdx.y, s = b * leaf;
+  const int size = (int)min((long long)leaf, n - s);
+  for (int c = blockIdx.x; c < size; c += gridDim.x)
+    for (int r = threadIdx.x; r < min(size, c / 32 * 32 + 32); r += blockDim.x)
+      W[b * wstride + r + (long long)c * ldw] =
+          r < c / 32 * 32 ? 0.0 : D[(s / 32 + c / 32) * 1024 + (r & 31) + 32 * (c & 31)];
+}
+
+// All levels of the inverses of `nleaf` leaves of at most `leaf` rows.
+template <class T>
+tb_status trtri_levels(const T* A, long long lda, long long n, int leaf, int nleaf, const double* D, double* W,
+                       long long ldg, __half* hi, __half* lo, long long ldw, long long wstride, cudaStream_t st) {
+  const int nsub = (int)((std::min<long long>(leaf, n) + 31) / 32);
+  for (int h = 1; h < nsub; h *= 2) {
+    const dim3 g((unsigned)((nsub + h - 1) / (2 * h) * h * h), (unsigned)nleaf);
+    if (h == 1) {
+      trtri_level_kernel<T, 2><<<g, kChainThreads, 0, st>>>(A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h);
+    } else {
+      trtri_level_kernel<T, 0><<<g, kChainThreads, 0, st>>>(A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h);
+      TB_CUDA_TRY(cudaGetLastError());
+      note_launch();
+      trtri_level_kernel<T, 1><<<g, kChainThreads, 0, st>>>(A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h);
+    }
+    TB_CUDA_TRY(cudaGetLastError());
+    note_launch();
+  }
+  return TB_SUCCESS;
 }
 
 
@@ -446,16 +589,6 @@ tb_status trsm_prep_launch(const PrepJobs& j, cudaStream_t st) {
     p.conv_blocks[k] = gx * gy;
     next += gx * gy;
   }
-  if (j.D && j.n > 0) {
-    p.A = j.A;
-    p.lda = j.lda;
-    p.n = j.n;
-    p.D = j.D;
-    p.unit = j.unit ? 1 : 0;
-    p.diag_base = next;
-    p.diag_blocks = ((j.n + 31) / 32 + 3) / 4;
-    next += p.diag_blocks;
-  }
   if (j.zero && j.nzero > 0) {
     p.zero = j.zero;
     p.nzero = j.nzero;
@@ -465,22 +598,35 @@ tb_status trsm_prep_launch(const PrepJobs& j, cudaStream_t st) {
   }
   if (next == 0) return TB_SUCCESS;
   if (next > 0x7fffffffLL) return TB_ERROR_NOT_SUPPORTED;
-  trsm_prep_kernel<<<(unsigned)next, kPrepThreads, p.diag_blocks > 0 ? kPrepDiagSmem : 0, st>>>(p);
+  trsm_prep_kernel<<<(unsigned)next, kPrepThreads, 0, st>>>(p);
   TB_CUDA_TRY(cudaGetLastError());
   note_launch();
   return TB_SUCCESS;
 }
 
-// Diagonal-block inverses of many triangular matrices in two launches.
+// Diagonal-block inverses of many triangular matrices: one launch for the
+// 32 x 32 blocks, then the doubling levels over the jobs that reach them
+// (`chain` sorted by size, largest first; level_jobs[l]: how many leaves have
+// more than 2^l sub-blocks).
 tb_status trsm_inverses_grouped(const DiagJob* d_diag, int ndiag, long long nblocks, const ChainJob* d_chain,
-                                int nchain, cudaStream_t st) {
+                                const std::vector<int>& level_jobs, cudaStream_t st) {
   if (ndiag > 0 && nblocks > 0) {
     diag_inv32_grouped_kernel<<<(unsigned)nblocks, 32, 0, st>>>(d_diag, ndiag);
     TB_CUDA_TRY(cudaGetLastError());
     note_launch();
   }
-  if (nchain > 0) {
-    trtri_chain_grouped_kernel<<<dim3(kLeafMax / 32, (unsigned)nchain), kChainThreads, 0, st>>>(d_chain);
+  for (size_t l = 0; l < level_jobs.size(); ++l) {
+    if (level_jobs[l] <= 0) break;
+    const int h = 1 << l;
+    const dim3 g((unsigned)((kLeafMax / 32 + h - 1) / (2 * h) * h * h), (unsigned)level_jobs[l]);
+    if (h == 1) {
+      trtri_level_grouped_kernel<2><<<g, kChainThreads, 0, st>>>(d_chain, h);
+    } else {
+      trtri_level_grouped_kernel<0><<<g, kChainThreads, 0, st>>>(d_chain, h);
+      TB_CUDA_TRY(cudaGetLastError());
+      note_launch();
+      trtri_level_grouped_kernel<1><<<g, kChainThreads, 0, st>>>(d_chain, h);
+    }
     TB_CUDA_TRY(cudaGetLastError());
     note_launch();
   }
@@ -488,19 +634,16 @@ tb_status trsm_inverses_grouped(const DiagJob* d_diag, int ndiag, long long nblo
 }
 
 // FP64 inverses of the diagonal leaf blocks of an FP64 lower-triangular
-// matrix (order nt): leaf b = {s_b, size_b} (s_b a multiple of 32, size_b <=
-// 512) gets W_b = inv(A[s_b:, s_b:]) at W + b * wstride (ld ldw, zeros above
-// the diagonal). D: (nt + 31) / 32 * 1024 doubles of scratch; d_leaves: the
-// leaves in device memory.
-tb_status trsm_leaf_inverses_f64(long nt, const double* A, long lda, const int2* d_leaves, int nleaf, int max_size,
-                                 double* D, double* W, long long ldw, long long wstride, cudaStream_t st, bool unit) {
-  const long nsub = (nt + 31) / 32;
-  diag_inv32_kernel<double><<<(unsigned)nsub, 32, 0, st>>>(nt, A, lda, D, unit);
-  TB_CUDA_TRY(cudaGetLastError());
-  note_launch();
-  const int max_chain = (max_size + 31) / 32;
-  trtri_chain_f64_kernel<<<dim3((unsigned)max_chain, (unsigned)nleaf), kChainThreads, 0, st>>>(A, lda, d_leaves, D, W,
-                                                                                              ldw, wstride);
+// matrix (order nt): leaf b, rows [b * leaf, ...) of at most `leaf` (a
+// multiple of 32, <= 512), gets W_b at W + b * wstride (ld ldw >= the leaf
+// rounded up to 32, zeros above the diagonal). D: (nt + 31) / 32 * 1024
+// doubles of scratch.
+tb_status trsm_leaf_inverses_f64(long nt, const double* A, long lda, int leaf, int nleaf, double* D, double* W,
+                                 long long ldw, long long wstride, cudaStream_t st, bool unit) {
+  TB_TRY(diag_inv32<double>(nt, A, lda, D, unit, WOut{}, st));
+  TB_TRY(trtri_levels<double>(A, lda, nt, leaf, nleaf, D, W, ldw, nullptr, nullptr, ldw, wstride, st));
+  trtri_finish_f64_kernel<<<dim3((unsigned)std::min<long>(leaf, nt), (unsigned)nleaf), 256, 0, st>>>(nt, leaf, D, W,
+                                                                                                    ldw, wstride);
   TB_CUDA_TRY(cudaGetLastError());
   note_launch();
   return TB_SUCCESS;
@@ -513,7 +656,7 @@ tb_status trsm_leaf_inverses_f64(long nt, const double* A, long lda, const int2*
 // take it from the pool.
 namespace {
 struct TrsmLayout {
-  size_t o_ah, o_al, o_xh, o_xl, o_wh, o_wl, o_rh, o_rl, o_d, o_lv, o_wg, total;
+  size_t o_ah, o_al, o_xh, o_xl, o_wh, o_wl, o_rh, o_rl, o_d, o_wg, total;
 };
 
 TrsmLayout trsm_layout(TrsmCtx& c, long nleaf) {
@@ -530,7 +673,6 @@ TrsmLayout trsm_layout(TrsmCtx& c, long nleaf) {
   const size_t w_bytes = (size_t)c.wstride * nleaf * 2;
   const size_t r_bytes = (size_t)c.ldr * (c.right ? c.leaf : c.n) * 2;
   const size_t d_bytes = (size_t)((nt + 31) / 32) * 1024 * sizeof(double);
-  const size_t l_bytes = (size_t)nleaf * sizeof(int2);
   TrsmLayout L;
   size_t off = 0;
   auto take = [&](size_t b) {
@@ -547,7 +689,6 @@ TrsmLayout trsm_layout(TrsmCtx& c, long nleaf) {
   L.o_rh = take(r_bytes);
   L.o_rl = take(r_bytes);
   L.o_d = take(d_bytes);
-  L.o_lv = take(l_bytes);
   L.o_wg = take((size_t)c.wstride * nleaf * sizeof(double));  // FP64 panels of the leaf inverses
   L.total = off;
   return L;
@@ -577,12 +718,8 @@ tb_status trsm_setup(bool right, long m, long n, const float* A, long lda, long 
   const bool hilo = c.split == Split::kHiLo;
 
   leaf_start.clear();
-  std::vector<int2> leaves;
-  for (long s = 0; s < nt; s += leaf) {
-    leaf_start.push_back(s);
-    leaves.push_back(make_int2((int)s, (int)std::min<long>(leaf, nt - s)));
-  }
-  const long nleaf = (long)leaves.size();
+  for (long s = 0; s < nt; s += leaf) leaf_start.push_back(s);
+  const long nleaf = (long)leaf_start.size();
   const TrsmLayout L = trsm_layout(c, nleaf);
   char* ws = static_cast<char*>(scratch ? scratch : pool_get(L.total));
   if (!ws) {
@@ -598,9 +735,7 @@ tb_status trsm_setup(bool right, long m, long n, const float* A, long lda, long 
   c.rh = reinterpret_cast<__half*>(ws + L.o_rh);
   c.rl = reinterpret_cast<__half*>(ws + L.o_rl);
   double* D = reinterpret_cast<double*>(ws + L.o_d);
-  int2* dleaves = reinterpret_cast<int2*>(ws + L.o_lv);
   double* W64 = reinterpret_cast<double*>(ws + L.o_wg);
-  TB_CUDA_TRY(cudaMemcpyAsync(dleaves, leaves.data(), nleaf * sizeof(int2), cudaMemcpyHostToDevice, st));
 
   // 1. on the caller's stream, one conversion launch: the FP16 copy of A's
   // lower part (only off-diagonal leaf blocks are read) and, when B is known,
@@ -635,7 +770,7 @@ tb_status trsm_setup(bool right, long m, long n, const float* A, long lda, long 
     c.r0_ready = true;
   }
   // 2. beside it, on an auxiliary stream: the 32 x 32 FP64 inverses of A's
-  // diagonal and the leaf chains (they read only A and each other), joined
+  // diagonal and the leaf inverses' levels (they read only A and each other), joined
   // back into the caller's stream before the solve
   const cudaStream_t sa = aux_stream(1);
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -648,20 +783,10 @@ tb_status trsm_setup(bool right, long m, long n, const float* A, long lda, long 
   if (sa && (cudaEventRecord(fork, st) != cudaSuccess || cudaStreamWaitEvent(sa, fork, 0) != cudaSuccess))
     rs = TB_ERROR_CUDA;
   if (rs == TB_SUCCESS) {
-    PrepJobs inv;
-    inv.A = A;
-    inv.lda = lda;
-    inv.n = nt;
-    inv.D = D;
-    inv.unit = unit;
-    rs = trsm_prep_launch(inv, si);
+    rs = diag_inv32<float>(nt, A, lda, D, unit, WOut{c.wh, c.wl, c.ldw, c.wstride, c.leaf}, si);
   }
   if (rs == TB_SUCCESS) {
-    const int max_chain = (int)(leaf / 32);
-    dim3 grid((unsigned)max_chain, (unsigned)nleaf);
-    trtri_chain_kernel<<<grid, kChainThreads, 0, si>>>(A, lda, dleaves, D, c.wh, c.wl, c.ldw, c.wstride, W64);
-    if (cudaGetLastError() != cudaSuccess) rs = TB_ERROR_CUDA;
-    note_launch();
+    rs = trtri_levels<float>(A, lda, nt, c.leaf, (int)nleaf, D, W64, c.ldw, c.wh, c.wl, c.ldw, c.wstride, si);
   }
   if (rs == TB_SUCCESS) rs = trsm_prep_launch(conv, st);
   if (sa && (cudaEventRecord(join, sa) != cudaSuccess || cudaStreamWaitEvent(st, join, 0) != cudaSuccess) &&
