@@ -24,6 +24,7 @@
 #include <cstring>
 #include <vector>
 
+#include "tb_convert.cuh"
 #include "tb_gemm.cuh"
 #include "tb_internal.h"
 
@@ -36,54 +37,33 @@ struct ConvJob {
   __half* hi;
   __half* lo;
   long long ldd;
-  int tri;
+  int tri, al;
   long long first;  // first block index of this job in the grouped launch
 };
 
-constexpr int kConvPerThread = 8;
-constexpr int kConvPerBlock = 256 * kConvPerThread;  // elements per block of the grouped conversion
+constexpr int kConvThreads = 256;
 
-// kConvPerBlock consecutive elements (column-major order over rows x cols)
-// of one job per block, so short columns of small instances do not leave
-// most of a block idle. blk_job maps a block to its job (one load, where a
-// search over the job table would be a chain of dependent loads per block);
-// each thread issues all its loads before it converts and stores.
-__global__ void __launch_bounds__(256) conv_grouped_kernel(const ConvJob* __restrict__ jobs,
-                                                           const int* __restrict__ blk_job) {
+// One group of up to 8 rows of a column per thread (16-byte stores into the
+// padded FP16 copies; 16-byte loads where the instance's columns are aligned),
+// groups in column-major order, so short columns of small instances do not
+// leave most of a block idle. blk_job maps a block to its job (one load, where
+// a search over the job table would be a chain of dependent loads per block).
+// One element per thread and 2-byte stores took 796 us for the 512-instance
+// batch, this 500 us.
+__global__ void __launch_bounds__(kConvThreads) conv_grouped_kernel(const ConvJob* __restrict__ jobs,
+                                                                    const int* __restrict__ blk_job) {
   const long long b = blockIdx.x;
   const ConvJob& jb = jobs[blk_job[b]];
-  const long long rows = jb.rows, total = jb.rows * jb.cols, lds = jb.lds, ldd = jb.ldd;
-  const float* const src = jb.src;
-  __half* const dhi = jb.hi;
-  __half* const dlo = jb.lo;
-  const int tri = jb.tri;
-  const long long e0 = (b - jb.first) * kConvPerBlock + threadIdx.x;
-  long long at[kConvPerThread];
-  float f[kConvPerThread];
-  // (i, j) of element e0 by one division; the thread's later elements step
-  // 256 further each, which moves i on and wraps it into the next column(s)
-  long long j = e0 / rows, i = e0 - j * rows;
-#pragma unroll
-  for (int q = 0; q < kConvPerThread; ++q) {
-    const long long e = e0 + q * 256;
-    if (q > 0) {
-      i += 256;
-      while (i >= rows) {
-        i -= rows;
-        ++j;
-      }
-    }
-    const bool ok = e < total && !(tri == 2 && i < ((j >> 3) << 3));
-    at[q] = ok ? i + j * ldd : -1;
-    f[q] = ok ? __ldg(src + i + j * lds) : 0.f;
-  }
-#pragma unroll
-  for (int q = 0; q < kConvPerThread; ++q) {
-    if (at[q] < 0) continue;
-    const __half h = __float2half_rn(f[q]);
-    dhi[at[q]] = h;
-    if (dlo) dlo[at[q]] = __float2half_rn((f[q] - __half2float(h)) * 2048.f);
-  }
+  const unsigned rows8 = (unsigned)((jb.rows + 7) >> 3);
+  const long long g = (b - jb.first) * kConvThreads + threadIdx.x;
+  if (g >= (long long)rows8 * jb.cols) return;
+  const unsigned j = (unsigned)g / rows8, v = (unsigned)g - j * rows8;  // groups of a job fit 32 bits (n <= 65536)
+  if (jb.tri == 2 && v < (j >> 3)) return;
+  const long long i = 8ll * v;
+  const int nv = (int)min(8LL, jb.rows - i);
+  float f[8];
+  conv::load8(jb.src + i + j * jb.lds, nv, jb.al != 0, f);
+  conv::store8(f, nv, jb.hi, jb.lo, i + j * jb.ldd, 0, 2048.f);
 }
 
 struct Launch {
@@ -327,8 +307,8 @@ extern "C" tb_status tb_batch_create(tb_batch_t* out, int count, const int* kind
   long long conv_nblk = 0, diag_blocks = 0;
   auto add_conv = [&](const float* src, long long rows, long long cols, long long lds, __half* hi, __half* lo,
                       long long ldd, int tri) {
-    conv.push_back(ConvJob{src, rows, cols, lds, hi, lo, ldd, tri, conv_nblk});
-    conv_nblk += (rows * cols + kConvPerBlock - 1) / kConvPerBlock;
+    conv.push_back(ConvJob{src, rows, cols, lds, hi, lo, ldd, tri, conv::convert_aligned(src, lds) ? 1 : 0, conv_nblk});
+    conv_nblk += ((rows + 7) / 8 * cols + kConvThreads - 1) / kConvThreads;
   };
   for (SyrkPlan& s : syrks) {
     add_conv(s.A, s.n, s.n, s.lda, H(s.off_h), hilo ? H(s.off_l) : nullptr, s.ldh, 0);
@@ -503,7 +483,7 @@ extern "C" tb_status tb_batch_run(tb_batch_t b) {
   cudaStream_t st = current_stream();
   if (b->nconv > 0 && b->conv_blocks > 0) {
     if (b->conv_blocks > 0x7fffffffLL) return TB_ERROR_NOT_SUPPORTED;
-    conv_grouped_kernel<<<(unsigned)b->conv_blocks, 256, 0, st>>>(b->d_conv, b->d_blk_job);
+    conv_grouped_kernel<<<(unsigned)b->conv_blocks, kConvThreads, 0, st>>>(b->d_conv, b->d_blk_job);
     TB_CUDA_TRY(cudaGetLastError());
     note_launch();
   }

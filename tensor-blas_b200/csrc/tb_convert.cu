@@ -14,15 +14,16 @@ namespace tb {
 
 namespace {
 
-// Vector path: rows % 8 == 0, lds % 4 == 0, ldd % 8 == 0, 16-byte aligned bases.
+// Vector path (convert8_body).
 __global__ void __launch_bounds__(256) convert8_kernel(long long rows, long long cols, const float* __restrict__ src,
-                                                       long long lds, __half* __restrict__ hi, __half* __restrict__ lo,
-                                                       long long ldd, float lo_scale, int tri, long long dup) {
-  conv::convert8_body(blockIdx.x, gridDim.x, blockIdx.y, gridDim.y, rows, cols, src, lds, hi, lo, ldd, lo_scale, tri,
-                      dup);
+                                                       long long lds, int al, __half* __restrict__ hi,
+                                                       __half* __restrict__ lo, long long ldd, float lo_scale, int tri,
+                                                       long long dup) {
+  conv::convert8_body(blockIdx.x, gridDim.x, blockIdx.y, gridDim.y, rows, cols, src, lds, al != 0, hi, lo, ldd,
+                      lo_scale, tri, dup);
 }
 
-// Scalar fallback for ragged or unaligned shapes.
+// Scalar fallback for destinations that 16-byte stores cannot address.
 __global__ void __launch_bounds__(256) convert1_kernel(long long rows, long long cols, const float* __restrict__ src,
                                                        long long lds, __half* __restrict__ hi, __half* __restrict__ lo,
                                                        long long ldd, float lo_scale, int tri, long long dup) {
@@ -80,15 +81,13 @@ tb_status convert_sym_f32_f16(long long n, const float* A, long long lda, bool l
 tb_status convert_f32_f16(long long rows, long long cols, const float* src, long long lds, __half* hi, __half* lo,
                           long long ldd, float lo_scale, int tri, cudaStream_t stream, long long dup) {
   if (rows <= 0 || cols <= 0) return TB_SUCCESS;
-  const bool vec = (rows % 8 == 0) && (lds % 4 == 0) && (ldd % 8 == 0) &&
-                   (reinterpret_cast<uintptr_t>(src) % 16 == 0) && (reinterpret_cast<uintptr_t>(hi) % 16 == 0) &&
-                   (lo == nullptr || reinterpret_cast<uintptr_t>(lo) % 16 == 0);
+  const bool vec = conv::convert_vec(hi, lo, ldd, dup);
   const int threads = 256;
   long long gx = 0, gy = 0;
   conv::convert_grid(rows, cols, tri, vec, sm_count(), threads, &gx, &gy);
   dim3 grid((unsigned)gx, (unsigned)gy);
   if (vec)
-    convert8_kernel<<<grid, threads, 0, stream>>>(rows, cols, src, lds, hi, lo, ldd, lo_scale, tri, dup);
+    convert8_kernel<<<grid, threads, 0, stream>>>(rows, cols, src, lds, conv::convert_aligned(src, lds) ? 1 : 0, hi, lo, ldd, lo_scale, tri, dup);
   else
     convert1_kernel<<<grid, threads, 0, stream>>>(rows, cols, src, lds, hi, lo, ldd, lo_scale, tri, dup);
   TB_CUDA_TRY(cudaGetLastError());

@@ -27,13 +27,41 @@ __device__ __forceinline__ uint32_t pack2(__half a, __half b) {
 // other triangle only within 256 of the diagonal.
 constexpr long long kTriBand = 256;
 
-// Eight converted values of one column to hi (and lo), and their copies `dup`
-// elements further on.
-__device__ __forceinline__ void store8(const float* f, __half* __restrict__ hi, __half* __restrict__ lo,
+// Up to eight (nv) consecutive values of one column; al: 16-byte aligned.
+// Columns that are not are read as eight 4-byte loads a thread, whose sectors
+// the warp's later loads find in L1.
+__device__ __forceinline__ void load8(const float* s, int nv, bool al, float* f) {
+  if (nv == 8 && al) {
+    const float4 a = ld_stream(s), b = ld_stream(s + 4);
+    f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w;
+    f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] = e < nv ? __ldg(s + e) : 0.f;
+  }
+}
+
+// nv converted values of one column to hi (and lo), and their copies `dup`
+// elements further on; elements beyond nv are not touched.
+__device__ __forceinline__ void store8(const float* f, int nv, __half* __restrict__ hi, __half* __restrict__ lo,
                                        long long off, long long dup, float lo_scale) {
   __half h[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) h[e] = __float2half_rn(f[e]);
+  if (nv < 8) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      if (e >= nv) break;
+      hi[off + e] = h[e];
+      if (dup) hi[off + dup + e] = h[e];
+      if (lo) {
+        const __half l = __float2half_rn((f[e] - __half2float(h[e])) * lo_scale);
+        lo[off + e] = l;
+        if (dup) lo[off + dup + e] = l;
+      }
+    }
+    return;
+  }
   uint4 o;
   o.x = pack2(h[0], h[1]);
   o.y = pack2(h[2], h[3]);
@@ -55,88 +83,66 @@ __device__ __forceinline__ void store8(const float* f, __half* __restrict__ hi, 
   }
 }
 
-// Vector path: rows % 8 == 0, lds % 4 == 0, ldd % 8 == 0, 16-byte aligned bases.
-// Whole matrices (tri 0): a thread owns 8 rows and walks the columns by,
-// by + gy, ... four at a time, with the four columns' loads (128 bytes) in
-// flight together; grids of a few blocks per SM then keep enough bytes in
-// flight to run at the HBM rate.
+// Vector path: a thread owns 8 rows of a column (the last group of a column
+// may be shorter) and writes them with 16-byte stores: ldd a multiple of 8,
+// 16-byte aligned hi and lo. al: the source's columns are 16-byte aligned
+// (lds a multiple of 4). Ragged and unaligned sources took a one-row-per-thread
+// path before: A's lower part and the first leaf's 6003 x 512 rows of a TRSM
+// of order 4100 went from 277 to 37 us.
+// Whole matrices (tri 0): a thread walks the columns by, by + gy, ... four at
+// a time, with the four columns' loads (128 bytes) in flight together; grids
+// of a few blocks per SM then keep enough bytes in flight to run at the HBM
+// rate.
 __device__ __forceinline__ void convert8_body(long long bx, long long gx, long long by, long long gy, long long rows,
-                                              long long cols, const float* __restrict__ src, long long lds,
+                                              long long cols, const float* __restrict__ src, long long lds, bool al,
                                               __half* __restrict__ hi, __half* __restrict__ lo, long long ldd,
                                               float lo_scale, int tri, long long dup) {
-  const long long rows8 = rows >> 3;
+  const long long rows8 = (rows + 7) >> 3;
+  // rows [8v, ...) of the columns by, by + gy, ... below jend
+  auto walk = [&](long long v, long long jend) {
+    const long long i = v << 3;
+    const int nv = (int)min(8LL, rows - i);
+    long long j = by;
+    for (; j + 3 * gy < jend; j += 4 * gy) {
+      float f[4][8];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) load8(src + i + (j + u * gy) * lds, nv, al, f[u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) store8(f[u], nv, hi, lo, i + (j + u * gy) * ldd, dup, lo_scale);
+    }
+    for (; j < jend; j += gy) {
+      float f[8];
+      load8(src + i + j * lds, nv, al, f);
+      store8(f, nv, hi, lo, i + j * ldd, dup, lo_scale);
+    }
+  };
   if (tri == 2) {
     // lower part: row group v (rows 8v .. 8v + 7) has the columns j < 8v + 8.
     // A thread takes row groups t and rows8 - 1 - t, so every thread has
-    // about the same number of columns, and walks them four at a time.
+    // about the same number of columns.
     const long long half = (rows8 + 1) >> 1;
     for (long long t = bx * blockDim.x + threadIdx.x; t < half; t += gx * blockDim.x) {
       for (int w = 0; w < 2; ++w) {
         const long long v = w ? rows8 - 1 - t : t;
         if (w && v == t) break;
-        const long long i = v << 3, jend = min(cols, i + 8);
-        long long j = by;
-        for (; j + 3 * gy < jend; j += 4 * gy) {
-          float4 a[4], b[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float* s = src + i + (j + u * gy) * lds;
-            a[u] = ld_stream(s);
-            b[u] = ld_stream(s + 4);
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float f[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
-            store8(f, hi, lo, i + (j + u * gy) * ldd, dup, lo_scale);
-          }
-        }
-        for (; j < jend; j += gy) {
-          const float* s = src + i + j * lds;
-          const float4 a = ld_stream(s), b = ld_stream(s + 4);
-          const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-          store8(f, hi, lo, i + j * ldd, dup, lo_scale);
-        }
+        walk(v, min(cols, (v << 3) + 8));
       }
     }
     return;
   }
   if (tri == 0) {
-    for (long long v = bx * blockDim.x + threadIdx.x; v < rows8; v += gx * blockDim.x) {
-      const long long i = v << 3;
-      long long j = by;
-      for (; j + 3 * gy < cols; j += 4 * gy) {
-        float4 a[4], b[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float* s = src + i + (j + u * gy) * lds;
-          a[u] = ld_stream(s);
-          b[u] = ld_stream(s + 4);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float f[8] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w};
-          store8(f, hi, lo, i + (j + u * gy) * ldd, dup, lo_scale);
-        }
-      }
-      for (; j < cols; j += gy) {
-        const float* s = src + i + j * lds;
-        const float4 a = ld_stream(s), b = ld_stream(s + 4);
-        const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-        store8(f, hi, lo, i + j * ldd, dup, lo_scale);
-      }
-    }
+    for (long long v = bx * blockDim.x + threadIdx.x; v < rows8; v += gx * blockDim.x) walk(v, cols);
     return;
   }
   for (long long j = by; j < cols; j += gy) {
     long long v0 = bx * blockDim.x + threadIdx.x, vend = rows8;
-    if (tri == 2) v0 += (j >> 3);  // rows i >= j (rounded down to 8)
     if (tri == 4) vend = min(rows8, (j / kTriBand + 1) * (kTriBand / 8));  // rows i < band end
     if (tri == 5) v0 += (j / kTriBand) * (kTriBand / 8);                   // rows i >= band start
     for (long long v = v0; v < vend; v += gx * blockDim.x) {
       const long long i = v << 3;
-      const float* s = src + i + j * lds;
-      const float4 a = ld_stream(s), b = ld_stream(s + 4);
-      float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      const int nv = (int)min(8LL, rows - i);
+      float f[8];
+      load8(src + i + j * lds, nv, al, f);
       if (tri == 1 || tri == 5) {
 #pragma unroll
         for (int e = 0; e < 8; ++e)
@@ -146,9 +152,18 @@ __device__ __forceinline__ void convert8_body(long long bx, long long gx, long l
         for (int e = 0; e < 8; ++e)
           if (i + e > j) f[e] = 0.f;
       }
-      store8(f, hi, lo, i + j * ldd, dup, lo_scale);
+      store8(f, nv, hi, lo, i + j * ldd, dup, lo_scale);
     }
   }
+}
+
+// Whether a conversion can take convert8_body, and with aligned loads.
+inline bool convert_vec(const void* hi, const void* lo, long long ldd, long long dup) {
+  return ldd % 8 == 0 && dup % 8 == 0 && reinterpret_cast<uintptr_t>(hi) % 16 == 0 &&
+         reinterpret_cast<uintptr_t>(lo) % 16 == 0;
+}
+inline bool convert_aligned(const void* src, long long lds) {
+  return lds % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
 }
 
 // Grid (gx, gy) of convert8_body / convert1_body for a rows x cols operand:
@@ -157,7 +172,7 @@ __device__ __forceinline__ void convert8_body(long long bx, long long gx, long l
 // column per block row.
 inline void convert_grid(long long rows, long long cols, int tri, bool vec, int sms, int threads, long long* gx,
                          long long* gy) {
-  long long units = vec ? rows / 8 : rows;
+  long long units = vec ? (rows + 7) / 8 : rows;
   if (vec && tri == 2) units = (units + 1) / 2;  // two row groups per thread
   long long x = (units + threads - 1) / threads;
   if (x > 1024) x = 1024;
@@ -171,7 +186,7 @@ inline void convert_grid(long long rows, long long cols, int tri, bool vec, int 
   *gy = y;
 }
 
-// Scalar fallback for ragged or unaligned shapes.
+// Scalar fallback for destinations that 16-byte stores cannot address.
 __device__ __forceinline__ void convert1_body(long long bx, long long gx, long long by, long long gy, long long rows,
                                               long long cols, const float* __restrict__ src, long long lds,
                                               __half* __restrict__ hi, __half* __restrict__ lo, long long ldd,

@@ -156,7 +156,7 @@ tb_status diag_inv32(long long n, const T* A, long long lda, double* D, bool uni
 // arithmetic).
 struct PrepDev {
   PrepConv conv[2];
-  int conv_vec[2];
+  int conv_vec[2];  // 0: element by element, 1: 16-byte stores, 2: and 16-byte loads
   long long conv_gx[2], conv_base[2], conv_blocks[2];
   int nconv;
   int* zero;
@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(kPrepThreads) trsm_prep_kernel(const __grid_co
       const long long gy = p.conv_blocks[z] / gx;
       const PrepConv& c = p.conv[z];
       if (p.conv_vec[z])
-        conv::convert8_body(local % gx, gx, local / gx, gy, c.rows, c.cols, c.src, c.lds, c.hi, c.lo, c.ldd, 2048.f,
-                            c.tri, 0);
+        conv::convert8_body(local % gx, gx, local / gx, gy, c.rows, c.cols, c.src, c.lds, p.conv_vec[z] == 2, c.hi,
+                            c.lo, c.ldd, 2048.f, c.tri, 0);
       else
         conv::convert1_body(local % gx, gx, local / gx, gy, c.rows, c.cols, c.src, c.lds, c.hi, c.lo, c.ldd, 2048.f,
                             c.tri, 0);
@@ -578,12 +578,10 @@ tb_status trsm_prep_launch(const PrepJobs& j, cudaStream_t st) {
     const int k = p.nconv++;
     p.conv[k] = c;
     // the grid the conversion kernels would use (tb_convert.cu)
-    const bool vec = (c.rows % 8 == 0) && (c.lds % 4 == 0) && (c.ldd % 8 == 0) &&
-                     (reinterpret_cast<uintptr_t>(c.src) % 16 == 0) && (reinterpret_cast<uintptr_t>(c.hi) % 16 == 0) &&
-                     (c.lo == nullptr || reinterpret_cast<uintptr_t>(c.lo) % 16 == 0);
+    const bool vec = conv::convert_vec(c.hi, c.lo, c.ldd, 0);
     long long gx = 0, gy = 0;
     conv::convert_grid(c.rows, c.cols, c.tri, vec, sm_count(), kPrepThreads, &gx, &gy);
-    p.conv_vec[k] = vec ? 1 : 0;
+    p.conv_vec[k] = vec ? (conv::convert_aligned(c.src, c.lds) ? 2 : 1) : 0;
     p.conv_gx[k] = gx;
     p.conv_base[k] = next;
     p.conv_blocks[k] = gx * gy;
