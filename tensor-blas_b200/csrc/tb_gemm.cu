@@ -440,7 +440,14 @@ static std::vector<int4> merge_pairs(const std::vector<int4>& plan, int M, int N
 
 tb_status gemm_launch_plan(GemmCall& c, const std::vector<int4>& plan, cudaStream_t stream) {
   const bool pf = c.kblocks > 0 && c.kblocks <= kGemmPfMaxKb;
-  c.pair = !pf && c.M >= 512 && c.N >= 512 && pair_engine_enabled() &&
+  // short plain launches: pairs halve the operand bytes a flop takes, which is
+  // what bounds them once they fill the SMs, but a pair tile takes longer than
+  // a 128 x 128 one. C -= A B on a B200, single / pair: 1024 x 16384 x 1024 59 /
+  // 45 us, 1024 x 4096 x 1024 22.6 / 20.5, 1024 x 2048 x 1024 (128 tiles on 148
+  // SMs) 16.4 / 20.5; 512 x 16384 x 512 24.6 / 24.6, 512 x 4096 x 512 14.4 / 16.4
+  const bool short_pair = pf && !c.fp8 && c.split == Split::kPlain && c.kblocks > kGemmPfMaxKb / 2 &&
+                          (int)plan.size() > sm_count();
+  c.pair = (!pf || short_pair) && c.M >= 512 && c.N >= 512 && pair_engine_enabled() &&
            (c.fp8 || c.split == Split::kPlain || pair_split_enabled());
   std::vector<int4> merged;
   if (c.pair) {
