@@ -111,28 +111,32 @@ bool make_c_map(CUtensorMap* map, float* C, long long rows, long long cols, long
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// TB_PDL=1 in the environment launches the GEMM engine's kernels with
-// programmatic stream serialization (read once): a launch's CTAs may take
-// the SMs that the previous grid on the stream frees during its last tiles
-// and run their set-up (barriers, TMEM allocation) there, then wait in
-// grid_dep_wait until that grid has completed. Off by default: on a B200
-// the plain TRSM m = n = 16384 (nb 512, 63 dependent launches) took
-// 6.11 ms with it against 6.04 ms without, SYRK 16384 3.48 ms either way,
-// with identical results. Launches into a stream under graph capture are
-// always plain.
-static bool pdl_enabled() {
+}  // namespace
+
+// Programmatic stream serialization: a launch's CTAs may start while the
+// previous grid on the stream still runs (once all of its CTAs have started),
+// do their set-up (barriers, TMEM allocation) and wait in grid_dep_wait until
+// that grid has completed. Chains of short launches gain most: on a B200 the
+// TRSM of 4096 x 256 (nb 256, 31 launches) took 483 us without it and 451
+// with, 4096 x 4096 (nb 512) 432 / 405, 8192 x 8192 1210 / 1151; order 16384 is
+// the same within the runs' spread. TB_PDL=0 in the environment (read once)
+// turns it off, with the same results. Launches into a stream under graph
+// capture are always plain.
+bool dependent_launch(cudaStream_t stream) {
   static const bool on = [] {
     const char* e = getenv("TB_PDL");
-    return e && e[0] == '1';
+    return !(e && e[0] == '0');
   }();
-  return on;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return on && cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
 }
+
+namespace {
 
 template <class K>
 static cudaError_t launch_engine(K* kernel, unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
                                  const GemmArgs& args) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (pdl_enabled() && cudaStreamIsCapturing(stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
+  if (dependent_launch(stream)) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);

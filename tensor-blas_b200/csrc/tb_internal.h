@@ -140,6 +140,9 @@ int gemm_bn(Split s);
 int gemm_bn(Split s, int kblocks);
 
 tb_status gemm_launch(GemmCall& call, cudaStream_t stream);
+// Whether kernels that wait in grid_dep_wait may be launched with programmatic
+// stream serialization on this stream.
+bool dependent_launch(cudaStream_t stream);
 // GEMM engine for the large plain launches of this thread: -1 the default
 // (CTA pairs unless TB_GEMM_PAIR=0), 0 single-CTA 128 x 256 tiles, 1 CTA
 // pairs (256 x 256), 2 single-CTA 128 x 128 tiles (kEngineNarrow: twice the

@@ -27,6 +27,7 @@
 
 #include "tb_convert.cuh"
 #include "tb_internal.h"
+#include "tb_ptx.cuh"
 
 namespace tb {
 
@@ -383,6 +384,8 @@ template <class T, int PHASE>
 __global__ void __launch_bounds__(kChainThreads)
     trtri_level_kernel(const T* __restrict__ A, long long lda, long long n, int leaf, const double* __restrict__ D,
                        double* W, long long ldg, __half* hi, __half* lo, long long ldw, long long wstride, int h) {
+  grid_dep_launch();
+  grid_dep_wait();  // the previous level (or the diagonal inverses) is complete
   const long long b = blockIdx.y, s = b * leaf;
   LeafRef f;
   f.A = A + s + s * lda;
@@ -400,6 +403,8 @@ __global__ void __launch_bounds__(kChainThreads)
 // Grouped form: one job per (instance, leaf) along blockIdx.y, largest first.
 template <int PHASE>
 __global__ void __launch_bounds__(kChainThreads) trtri_level_grouped_kernel(const ChainJob* __restrict__ jobs, int h) {
+  grid_dep_launch();
+  grid_dep_wait();
   const ChainJob& jb = jobs[blockIdx.y];
   LeafRef f;
   f.A = jb.A + jb.s + (long long)jb.s * jb.lda;
@@ -427,6 +432,25 @@ __global__ void __launch_bounds__(256) trtri_finish_f64_kernel(long long n, int 
           r < c / 32 * 32 ? 0.0 : D[(s / 32 + c / 32) * 1024 + (r & 31) + 32 * (c & 31)];
 }
 
+// A kernel that waits in grid_dep_wait before it reads the previous launch's
+// results: its CTAs start as that launch's finish (a level's launch is 5 to 10
+// us, about two of them launch latency).
+template <class... P, class... Args>
+tb_status launch_level(void (*kernel)(P...), dim3 grid, cudaStream_t st, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kChainThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = dependent_launch(st) ? 1 : 0;
+  TB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+  note_launch();
+  return TB_SUCCESS;
+}
+
 // All levels of the inverses of `nleaf` leaves of at most `leaf` rows.
 template <class T>
 tb_status trtri_levels(const T* A, long long lda, long long n, int leaf, int nleaf, const double* D, double* W,
@@ -435,15 +459,11 @@ tb_status trtri_levels(const T* A, long long lda, long long n, int leaf, int nle
   for (int h = 1; h < nsub; h *= 2) {
     const dim3 g((unsigned)((nsub + h - 1) / (2 * h) * h * h), (unsigned)nleaf);
     if (h == 1) {
-      trtri_level_kernel<T, 2><<<g, kChainThreads, 0, st>>>(A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h);
+      TB_TRY(launch_level(trtri_level_kernel<T, 2>, g, st, A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h));
     } else {
-      trtri_level_kernel<T, 0><<<g, kChainThreads, 0, st>>>(A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h);
-      TB_CUDA_TRY(cudaGetLastError());
-      note_launch();
-      trtri_level_kernel<T, 1><<<g, kChainThreads, 0, st>>>(A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h);
+      TB_TRY(launch_level(trtri_level_kernel<T, 0>, g, st, A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h));
+      TB_TRY(launch_level(trtri_level_kernel<T, 1>, g, st, A, lda, n, leaf, D, W, ldg, hi, lo, ldw, wstride, h));
     }
-    TB_CUDA_TRY(cudaGetLastError());
-    note_launch();
   }
   return TB_SUCCESS;
 }
@@ -618,15 +638,11 @@ tb_status trsm_inverses_grouped(const DiagJob* d_diag, int ndiag, long long nblo
     const int h = 1 << l;
     const dim3 g((unsigned)((kLeafMax / 32 + h - 1) / (2 * h) * h * h), (unsigned)level_jobs[l]);
     if (h == 1) {
-      trtri_level_grouped_kernel<2><<<g, kChainThreads, 0, st>>>(d_chain, h);
+      TB_TRY(launch_level(trtri_level_grouped_kernel<2>, g, st, d_chain, h));
     } else {
-      trtri_level_grouped_kernel<0><<<g, kChainThreads, 0, st>>>(d_chain, h);
-      TB_CUDA_TRY(cudaGetLastError());
-      note_launch();
-      trtri_level_grouped_kernel<1><<<g, kChainThreads, 0, st>>>(d_chain, h);
+      TB_TRY(launch_level(trtri_level_grouped_kernel<0>, g, st, d_chain, h));
+      TB_TRY(launch_level(trtri_level_grouped_kernel<1>, g, st, d_chain, h));
     }
-    TB_CUDA_TRY(cudaGetLastError());
-    note_launch();
   }
   return TB_SUCCESS;
 }
