@@ -406,15 +406,17 @@ __device__ __forceinline__ void pick16(const float (&acc)[N], int c, float* v) {
 // Whether a tile's chunks go through the C slots (TMA); the others are
 // stored per element. Masked tiles with beta == 0 store their unmasked
 // elements directly: the slots would first have to load C to keep the masked
-// ones.
-__device__ __forceinline__ bool tile_staged(const GemmArgs& P, bool masked) {
-  return P.tma_c && !(masked && P.beta == 0.0f);
+// ones. TMA stores clip at 16 bytes, not at the element: the last row tile of
+// a C whose M is no multiple of 4 is stored per element, or up to three rows
+// past M would be overwritten.
+__device__ __forceinline__ bool tile_staged(const GemmArgs& P, bool masked, int m0) {
+  return P.tma_c && !(masked && P.beta == 0.0f) && ((P.M & 3) == 0 || m0 + 128 <= P.M);
 }
 
 // Whether a tile's chunks pass through the C slots at all: also per-element
 // tiles that make side copies, which build them from the slot.
-__device__ __forceinline__ bool tile_slots(const GemmArgs& P, bool masked) {
-  return tile_staged(P, masked) || (P.out_hi && !masked);
+__device__ __forceinline__ bool tile_slots(const GemmArgs& P, bool masked, int m0) {
+  return tile_staged(P, masked, m0) || (P.out_hi && !masked);
 }
 
 // The C loader's walk (one thread): the CTA's tiles in the epilogue's chunk
@@ -437,8 +439,8 @@ struct CLoader {
   // chunks of the tile at (m0, n0) with gc columns per group; false when a wait gave up
   __device__ __forceinline__ bool tile(const GemmArgs& P, int m0, int n0, int gc, bool masked,
                                        volatile int* abort_flag) {
-    if (!tile_slots(P, masked)) return true;
-    const bool need = P.beta != 0.0f && P.tma_c;
+    if (!tile_slots(P, masked, m0)) return true;
+    const bool need = P.beta != 0.0f && tile_staged(P, masked, m0);
     for (int c0 = 0; c0 < gc; c0 += kEpiCols) {
 #pragma unroll
       for (int g = 0; g < kEpiGroups; ++g) {
@@ -559,8 +561,8 @@ __device__ __forceinline__ bool epilogue_tile(const GemmArgs& P, Group& g, Acc& 
   const int nval = min(max((sk.N - gy + kEpiCols - 1) / kEpiCols, 0), GC / kEpiCols);  // chunks inside C
   const bool side_vec = sk.side_vec();
   // kSlots false: no ring (launches that read no C and make no side copies)
-  const bool staged = Group::kSlots && m0 < P.M && tile_staged(P, masked);
-  const bool through = Group::kSlots && m0 < P.M && tile_slots(P, masked);
+  const bool staged = Group::kSlots && m0 < P.M && tile_staged(P, masked, m0);
+  const bool through = Group::kSlots && m0 < P.M && tile_slots(P, masked, m0);
   // per-element path: C's old values are loaded one chunk ahead, the first
   // before the accumulator wait (where the fold leaves registers for it)
   float old[kEpiCols];

@@ -828,7 +828,7 @@ size_t trsm_scratch_bytes(bool right, long m, long n, long nb, Split split) {
 // one persistent launch for all the recursion's products where B's layout
 // allows it (tb_trsm_dag.cu), else one GEMM launch per leaf and update.
 tb_status trsm_solve(TrsmCtx& c, const std::vector<long>& leaf_start, float* B, long ldb, long rows, long cols) {
-  if (trsm_dag_eligible(c, B, ldb)) return trsm_solve_dag(c, leaf_start, B, ldb, rows, cols);
+  if (rows % 4 == 0 && trsm_dag_eligible(c, B, ldb)) return trsm_solve_dag(c, leaf_start, B, ldb, rows, cols);
   return trsm_solve_launches(c, leaf_start, B, ldb, rows, cols);
 }
 
@@ -860,7 +860,7 @@ tb_status trsm_solve_2s(TrsmCtx& c, const std::vector<long>& leaf_start, float* 
     const int v = e ? atoi(e) : 0;
     return (v >= 1 && v <= 4) ? v : 1;
   }();
-  if (trsm_dag_eligible(c, B, ldb)) return trsm_solve_dag(c, leaf_start, B, ldb, rows, cols);
+  if (rows % 4 == 0 && trsm_dag_eligible(c, B, ldb)) return trsm_solve_dag(c, leaf_start, B, ldb, rows, cols);
   int parts = (c.split == Split::kPlain && span >= 4096) ? streams : 1;
   cudaStream_t sq[4] = {c.st, nullptr, nullptr, nullptr};
   for (int p = 1; p < parts; ++p)

@@ -935,7 +935,8 @@ bool trsm_dag_enabled() {
 bool trsm_dag_eligible(const TrsmCtx& c, const float* B, long ldb) {
   if (!trsm_dag_enabled()) return false;
   // TMA epilogue for every tile: C base 16-byte aligned, ldb a multiple of 4
-  if ((reinterpret_cast<uintptr_t>(B) & 15) != 0 || (ldb % 4) != 0) return false;
+  // and (TMA stores clip at 16 bytes) so is B's row count
+  if ((reinterpret_cast<uintptr_t>(B) & 15) != 0 || (ldb % 4) != 0 || (c.m % 4) != 0) return false;
   // at least two leaves (one leaf is a single product) and an order the
   // plain form solves in FP16 (smaller ones take the split path anyway)
   return c.nt > c.leaf;
