@@ -227,7 +227,7 @@ int gemm_bn(Split s, int kblocks) {
 tb_status gemm_build_args(const GemmCall& c, GemmArgs* out) {
   const bool split = c.split == Split::kHiLo && !c.fp8;
   // pair launches: each CTA loads half of the tile's B rows (128 of 256)
-  const int bn = c.fp8 ? kGemmBNFp8 : (c.pair ? 128 : gemm_bn(c.split, c.kblocks));
+  const int bn = c.fp8 ? kGemmBNFp8 : (c.pair ? 128 : (c.bn ? c.bn : gemm_bn(c.split, c.kblocks)));
   GemmArgs& a = *out;
   memset(&a, 0, sizeof(a));
   if (c.fp8) {
@@ -326,10 +326,15 @@ tb_status gemm_launch(GemmCall& c, cudaStream_t stream) {
     TB_BY_LAYOUT(TB_PAIR, PairMode::kStaged);
   }
   const bool pf = c.kblocks > 0 && c.kblocks <= kGemmPfMaxKb;
+  const int bn = c.bn ? c.bn : gemm_bn(c.split, c.kblocks);
+  if (bn == 64) {
+    if (split) TB_BY_LAYOUT(TB_SINGLE, 64, 3, true);
+    TB_BY_LAYOUT(TB_SINGLE, 64, 1, true);
+  }
   if (split && pf) TB_BY_LAYOUT(TB_SINGLE, 128, 3, true);
   if (split) TB_BY_LAYOUT(TB_SINGLE, 128, 3, false);
   if (pf) TB_BY_LAYOUT(TB_SINGLE, 128, 1, true);
-  if (gemm_bn(c.split, c.kblocks) == 128) TB_BY_LAYOUT(TB_SINGLE, 128, 1, false);
+  if (bn == 128) TB_BY_LAYOUT(TB_SINGLE, 128, 1, false);
   TB_BY_LAYOUT(TB_SINGLE, 256, 1, false);
 #undef TB_SINGLE
 #undef TB_PAIR
@@ -463,10 +468,32 @@ tb_status gemm_launch_plan(GemmCall& c, const std::vector<int4>& plan, cudaStrea
                wp = ((long)merged.size() + sms / 2 - 1) / (sms / 2);
     if (!c.fp8 && c.split == Split::kHiLo && wp * 1.45 > (double)ws) c.pair = false;
   }
-  if (c.pair)
+  if (c.pair) {
     TB_TRY(set_tiles(c, merged, std::min<int>((int)merged.size(), sm_count() / 2), stream));
-  else
+    return gemm_launch(c, stream);
+  }
+  // launches that leave more than half of the SMs idle run on narrower tiles
+  // (down to 64 columns): more CTAs, each with less to load, multiply and
+  // store (TRSM 4096 x 256, nb 256: 439 -> 375 us; 96 x 320: 131 -> 119). Not
+  // under an engine the autotuner set.
+  c.bn = gemm_bn(c.split, c.kblocks);
+  if (!c.fp8 && engine_override() < 0) {
+    std::vector<int4> narrow = plan;
+    while (c.bn > 64 && (int)narrow.size() * 2 <= sm_count()) {
+      const int half = c.bn / 2;
+      std::vector<int4> next;
+      next.reserve(narrow.size() * 2);
+      for (const int4& t : narrow) {
+        next.push_back(make_int4(t.x, t.y, t.z, t.w));
+        if (t.y + half < c.N) next.push_back(make_int4(t.x, t.y + half, t.z, t.w));
+      }
+      narrow.swap(next);
+      c.bn = half;
+    }
+    TB_TRY(set_tiles(c, narrow, std::min<int>((int)narrow.size(), sm_count()), stream));
+  } else {
     TB_TRY(set_tiles(c, plan, std::min<int>((int)plan.size(), sm_count()), stream));
+  }
   return gemm_launch(c, stream);
 }
 

@@ -172,6 +172,8 @@ constexpr int kGemmThreads = 32 * (kEpiWarp0 + 4 * kEpiGroups);
 // FP8 variant: e4m3 K-major operands scaled per 128 x 128 block; the
 // accumulator is folded into fp32 registers after every 128-deep K block
 // with the product of the two blocks' scales.
+// BN = 64 variants serve launches that leave more than half of the SMs idle
+// with wider tiles (the small solves): twice the CTAs, half the epilogue.
 template <int BN_, int NSPLIT_, bool A_MN_, bool B_MN_, bool PF_ = false, bool FP8_ = false>
 struct GemmCfg {
   static constexpr bool PF = PF_;
@@ -187,7 +189,7 @@ struct GemmCfg {
   static constexpr int A_BYTES = BM * BK * ELEM;
   static constexpr int B_BYTES = BN * BK * ELEM;
   static constexpr int STAGE_BYTES = NOPS * (A_BYTES + B_BYTES);
-  static constexpr int STAGES = FP8 ? 6 : PF ? (SPLIT ? 3 : 4) : (SPLIT ? 3 : (BN == 128 ? 6 : 4));
+  static constexpr int STAGES = BN == 64 ? (SPLIT ? 4 : 6) : FP8 ? 6 : PF ? (SPLIT ? 3 : 4) : (SPLIT ? 3 : (BN == 128 ? 6 : 4));
   // TMEM: two main accumulators (alternating by round), then two corrections
   // (alternating by tile)
   static constexpr int CORR_COL = 2 * BN;
@@ -195,7 +197,7 @@ struct GemmCfg {
   static_assert(TMEM_COLS <= 512, "TMEM budget");
   static constexpr int GC = BN / kEpiGroups;              // columns of one epilogue group
   static constexpr int CHUNK_BYTES = 128 * kEpiCols * 4;  // one staged 128 x 16 fp32 chunk
-  static constexpr int C_SLOTS = PF && !SPLIT ? 6 : 2;  // per group
+  static constexpr int C_SLOTS = BN == 64 || (PF && SPLIT) ? 2 : PF ? 6 : 2;  // per group (BN = 64: all its chunks)
   static constexpr int GROUP_BYTES = C_SLOTS * CHUNK_BYTES;
   static constexpr int EPI_BYTES = kEpiGroups * GROUP_BYTES;
   static constexpr int BAR_BYTES = 512;

@@ -120,6 +120,7 @@ struct GemmCall {
   // blocks of 128, per-(128-row block, K block) scales (row-block-major,
   // scale_ld K blocks per row block); tiles 128 x 128.
   bool pair = false;  // set by gemm_launch_plan: 256 x 256 tiles on CTA pairs (cta_group::2)
+  int bn = 0;         // set by gemm_launch_plan: tile width of a single-CTA launch (0: gemm_bn(split, kblocks))
   int epi_cols = 32;  // columns of the TMA boxes the epilogue moves C and the side copies in
   bool fp8 = false;
   const float* scale_a = nullptr;
