@@ -62,8 +62,8 @@ __global__ void __launch_bounds__(kConvThreads) conv_grouped_kernel(const ConvJo
   const long long i = 8ll * v;
   const int nv = (int)min(8LL, jb.rows - i);
   float f[8];
-  conv::load8(jb.src + i + j * jb.lds, nv, jb.al != 0, f);
-  conv::store8(f, nv, jb.hi, jb.lo, i + j * jb.ldd, 0, 2048.f);
+  conv::load8<false>(jb.src + i + j * jb.lds, nv, jb.al != 0, f);
+  conv::store8<false>(f, nv, jb.hi, jb.lo, i + j * jb.ldd, 0, 2048.f);
 }
 
 struct Launch {

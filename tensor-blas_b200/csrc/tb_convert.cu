@@ -15,11 +15,12 @@ namespace tb {
 namespace {
 
 // Vector path (convert8_body).
+template <bool WHOLE>
 __global__ void __launch_bounds__(256) convert8_kernel(long long rows, long long cols, const float* __restrict__ src,
                                                        long long lds, int al, __half* __restrict__ hi,
                                                        __half* __restrict__ lo, long long ldd, float lo_scale, int tri,
                                                        long long dup) {
-  conv::convert8_body(blockIdx.x, gridDim.x, blockIdx.y, gridDim.y, rows, cols, src, lds, al != 0, hi, lo, ldd,
+  conv::convert8_body<WHOLE>(blockIdx.x, gridDim.x, blockIdx.y, gridDim.y, rows, cols, src, lds, al != 0, hi, lo, ldd,
                       lo_scale, tri, dup);
 }
 
@@ -86,8 +87,10 @@ tb_status convert_f32_f16(long long rows, long long cols, const float* src, long
   long long gx = 0, gy = 0;
   conv::convert_grid(rows, cols, tri, vec, sm_count(), threads, &gx, &gy);
   dim3 grid((unsigned)gx, (unsigned)gy);
-  if (vec)
-    convert8_kernel<<<grid, threads, 0, stream>>>(rows, cols, src, lds, conv::convert_aligned(src, lds) ? 1 : 0, hi, lo, ldd, lo_scale, tri, dup);
+  if (vec && conv::convert_whole(src, lds, rows))
+    convert8_kernel<true><<<grid, threads, 0, stream>>>(rows, cols, src, lds, 1, hi, lo, ldd, lo_scale, tri, dup);
+  else if (vec)
+    convert8_kernel<false><<<grid, threads, 0, stream>>>(rows, cols, src, lds, conv::convert_aligned(src, lds) ? 1 : 0, hi, lo, ldd, lo_scale, tri, dup);
   else
     convert1_kernel<<<grid, threads, 0, stream>>>(rows, cols, src, lds, hi, lo, ldd, lo_scale, tri, dup);
   TB_CUDA_TRY(cudaGetLastError());

@@ -29,9 +29,12 @@ constexpr long long kTriBand = 256;
 
 // Up to eight (nv) consecutive values of one column; al: 16-byte aligned.
 // Columns that are not are read as eight 4-byte loads a thread, whose sectors
-// the warp's later loads find in L1.
+// the warp's later loads find in L1. WHOLE: nv == 8 and al always hold, which
+// keeps the ragged code out of the kernel (a small conversion is bound by
+// fetching its code: 3.0 us against 4.7).
+template <bool WHOLE>
 __device__ __forceinline__ void load8(const float* s, int nv, bool al, float* f) {
-  if (nv == 8 && al) {
+  if (WHOLE || (nv == 8 && al)) {
     const float4 a = ld_stream(s), b = ld_stream(s + 4);
     f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w;
     f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
@@ -43,12 +46,13 @@ __device__ __forceinline__ void load8(const float* s, int nv, bool al, float* f)
 
 // nv converted values of one column to hi (and lo), and their copies `dup`
 // elements further on; elements beyond nv are not touched.
+template <bool WHOLE>
 __device__ __forceinline__ void store8(const float* f, int nv, __half* __restrict__ hi, __half* __restrict__ lo,
                                        long long off, long long dup, float lo_scale) {
   __half h[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) h[e] = __float2half_rn(f[e]);
-  if (nv < 8) {
+  if (!WHOLE && nv < 8) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       if (e >= nv) break;
@@ -93,6 +97,7 @@ __device__ __forceinline__ void store8(const float* f, int nv, __half* __restric
 // a time, with the four columns' loads (128 bytes) in flight together; grids
 // of a few blocks per SM then keep enough bytes in flight to run at the HBM
 // rate.
+template <bool WHOLE>
 __device__ __forceinline__ void convert8_body(long long bx, long long gx, long long by, long long gy, long long rows,
                                               long long cols, const float* __restrict__ src, long long lds, bool al,
                                               __half* __restrict__ hi, __half* __restrict__ lo, long long ldd,
@@ -106,14 +111,14 @@ __device__ __forceinline__ void convert8_body(long long bx, long long gx, long l
     for (; j + 3 * gy < jend; j += 4 * gy) {
       float f[4][8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) load8(src + i + (j + u * gy) * lds, nv, al, f[u]);
+      for (int u = 0; u < 4; ++u) load8<WHOLE>(src + i + (j + u * gy) * lds, nv, al, f[u]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) store8(f[u], nv, hi, lo, i + (j + u * gy) * ldd, dup, lo_scale);
+      for (int u = 0; u < 4; ++u) store8<WHOLE>(f[u], nv, hi, lo, i + (j + u * gy) * ldd, dup, lo_scale);
     }
     for (; j < jend; j += gy) {
       float f[8];
-      load8(src + i + j * lds, nv, al, f);
-      store8(f, nv, hi, lo, i + j * ldd, dup, lo_scale);
+      load8<WHOLE>(src + i + j * lds, nv, al, f);
+      store8<WHOLE>(f, nv, hi, lo, i + j * ldd, dup, lo_scale);
     }
   };
   if (tri == 2) {
@@ -142,7 +147,7 @@ __device__ __forceinline__ void convert8_body(long long bx, long long gx, long l
       const long long i = v << 3;
       const int nv = (int)min(8LL, rows - i);
       float f[8];
-      load8(src + i + j * lds, nv, al, f);
+      load8<WHOLE>(src + i + j * lds, nv, al, f);
       if (tri == 1 || tri == 5) {
 #pragma unroll
         for (int e = 0; e < 8; ++e)
@@ -152,7 +157,7 @@ __device__ __forceinline__ void convert8_body(long long bx, long long gx, long l
         for (int e = 0; e < 8; ++e)
           if (i + e > j) f[e] = 0.f;
       }
-      store8(f, nv, hi, lo, i + j * ldd, dup, lo_scale);
+      store8<WHOLE>(f, nv, hi, lo, i + j * ldd, dup, lo_scale);
     }
   }
 }
@@ -164,6 +169,10 @@ inline bool convert_vec(const void* hi, const void* lo, long long ldd, long long
 }
 inline bool convert_aligned(const void* src, long long lds) {
   return lds % 4 == 0 && reinterpret_cast<uintptr_t>(src) % 16 == 0;
+}
+// Its WHOLE form: aligned loads and no partial group.
+inline bool convert_whole(const void* src, long long lds, long long rows) {
+  return rows % 8 == 0 && convert_aligned(src, lds);
 }
 
 // Grid (gx, gy) of convert8_body / convert1_body for a rows x cols operand:

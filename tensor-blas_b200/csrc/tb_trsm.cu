@@ -157,7 +157,7 @@ tb_status diag_inv32(long long n, const T* A, long long lda, double* D, bool uni
 // arithmetic).
 struct PrepDev {
   PrepConv conv[2];
-  int conv_vec[2];  // 0: element by element, 1: 16-byte stores, 2: and 16-byte loads
+  int conv_vec[2];  // 0: element by element, 1: 16-byte stores, 2: and loads, 3: no ragged rows
   long long conv_gx[2], conv_base[2], conv_blocks[2];
   int nconv;
   int* zero;
@@ -173,9 +173,12 @@ __global__ void __launch_bounds__(kPrepThreads) trsm_prep_kernel(const __grid_co
       const long long local = b - p.conv_base[z], gx = p.conv_gx[z];
       const long long gy = p.conv_blocks[z] / gx;
       const PrepConv& c = p.conv[z];
-      if (p.conv_vec[z])
-        conv::convert8_body(local % gx, gx, local / gx, gy, c.rows, c.cols, c.src, c.lds, p.conv_vec[z] == 2, c.hi,
-                            c.lo, c.ldd, 2048.f, c.tri, 0);
+      if (p.conv_vec[z] == 3)
+        conv::convert8_body<true>(local % gx, gx, local / gx, gy, c.rows, c.cols, c.src, c.lds, true, c.hi, c.lo,
+                                  c.ldd, 2048.f, c.tri, 0);
+      else if (p.conv_vec[z])
+        conv::convert8_body<false>(local % gx, gx, local / gx, gy, c.rows, c.cols, c.src, c.lds, p.conv_vec[z] == 2,
+                                   c.hi, c.lo, c.ldd, 2048.f, c.tri, 0);
       else
         conv::convert1_body(local % gx, gx, local / gx, gy, c.rows, c.cols, c.src, c.lds, c.hi, c.lo, c.ldd, 2048.f,
                             c.tri, 0);
@@ -601,7 +604,7 @@ tb_status trsm_prep_launch(const PrepJobs& j, cudaStream_t st) {
     const bool vec = conv::convert_vec(c.hi, c.lo, c.ldd, 0);
     long long gx = 0, gy = 0;
     conv::convert_grid(c.rows, c.cols, c.tri, vec, sm_count(), kPrepThreads, &gx, &gy);
-    p.conv_vec[k] = vec ? (conv::convert_aligned(c.src, c.lds) ? 2 : 1) : 0;
+    p.conv_vec[k] = !vec ? 0 : conv::convert_whole(c.src, c.lds, c.rows) ? 3 : conv::convert_aligned(c.src, c.lds) ? 2 : 1;
     p.conv_gx[k] = gx;
     p.conv_base[k] = next;
     p.conv_blocks[k] = gx * gy;
