@@ -6,8 +6,8 @@
 // per-problem GEMM descriptors with their tensor maps, TRSM leaf inverses —
 // and tb_batch_run enqueues:
 //   1. one grouped FP32 -> FP16 conversion over all operand copies,
-//   2. one grouped 32x32 FP64 diagonal-inverse launch and one grouped leaf
-//      inverse (column-chain) launch for all TRSM instances,
+//   2. one grouped 32x32 FP64 diagonal-inverse launch and two grouped launches
+//      per doubling level of the leaf inverses for all TRSM instances,
 //   3. one grouped GEMM launch per step of the TRSM recursion, the SYRK
 //      instances riding on the first: every instance's recursion alternates
 //      leaf product / off-diagonal update (leaf, update, leaf, ...), so step p

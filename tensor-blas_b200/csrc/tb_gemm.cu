@@ -193,8 +193,8 @@ tb_status launch_variant(const GemmArgs& args, int num_tiles, cudaStream_t strea
 }  // namespace
 
 // 4 K-blocks (256-deep) between folds: at n = k = 16384 on a B200 the split
-// SYRK / TRSM took 12.51 / 16.43 ms with 2, 11.69 / 15.18 ms with 4 and
-// 11.22 / 14.01 ms with 8, at normwise errors vs FP64 of 2.8e-7 / 1.3e-7,
+// SYRK / TRSM of an earlier tile shape took 12.51 / 16.43 ms with 2, 11.69 /
+// 15.18 ms with 4 and 11.22 / 14.01 ms with 8, at normwise errors vs FP64 of 2.8e-7 / 1.3e-7,
 // 3.7e-7 / 1.6e-7 and 6.6e-7 / 2.4e-7; 4 keeps the 1e-6 target with margin
 // as K grows.
 int split_kchunk() {

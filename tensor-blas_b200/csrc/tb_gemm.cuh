@@ -1017,14 +1017,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
 // free. Buffer 0 is the main accumulator (one phase a round), buffer 1 the
 // correction (one phase a tile). Per 64-deep K block and SM the 256 x 256 tile
 // moves 64 KB into shared memory and 96 KB out of it for 1536 MMA cycles,
-// where 256 x 128 tiles (which left room to double-buffer) moved 96 + 144 KB
-// and kept the tensor pipe 65 % busy: SYR2K n = 16384, k = 4096 went from 6.0
+// where 256 x 128 tiles (which left room to double-buffer) moved 96 + 144 KB.
+// The tensor pipe is 93 % busy while the SM is active against 65 %: SYR2K n = 16384, k = 4096 went from 6.0
 // to 5.3 ms.
 // kFp8: e4m3 operands, one 128-deep K block a round (512 MMA cycles per SM),
 // the accumulators double-buffered and folded with the blocks' scales. The
-// fold, not the MMAs, bounds the round; single-CTA 128 x 128 tiles have 256 MMA
-// cycles a round and as long a fold for a quarter of the work a pair does:
-// SYMM 16384 went from 8.8 to 6.6 ms.
+// path of a round's signals (commit, fold, release, next MMAs) bounds it: the
+// tensor pipe is 38 % busy, and with three quarters of the fold's work left
+// out an 8192 launch still takes 555 us of its 676. Single-CTA 128 x 128 tiles have 256 MMA cycles a round
+// and as long a path for a quarter of the work a pair does: SYMM 16384 went
+// from 8.8 to 6.6 ms.
 // The fold modes keep 128 sums per epilogue thread: the first four warps give
 // registers to the epilogue's eight (setmaxnreg: 128 x 72 + 256 x 216 = 384 x
 // 168, the launch's allocation).

@@ -158,8 +158,9 @@ struct EngineScope {
   explicit EngineScope(int engine) : saved(engine_override()) { set_engine_override(engine); }
   ~EngineScope() { set_engine_override(saved); }
 };
-// Uploads `plan` (128-row tiles) and launches; plain launches that are large
-// enough run on CTA pairs, with the plan merged into 256-row tiles.
+// Uploads `plan` (128-row tiles) and launches; launches that are large enough
+// run on CTA pairs, with the plan merged into 256 x 256 tiles, and launches
+// that leave half the SMs idle on narrower tiles.
 tb_status gemm_launch_plan(GemmCall& call, const std::vector<int4>& plan, cudaStream_t stream);
 
 // Grouped launches: each problem's descriptor is built on the host by
@@ -268,7 +269,7 @@ struct TrsmCtx {
   // operand copy (rh / rl) from the B it was given
   bool r0_ready = false;
 };
-// Jobs of the one-launch TRSM preparation (trsm_prep_launch, tb_trsm.cu).
+// The TRSM's conversions and zeroed counters in one launch (trsm_prep_launch, tb_trsm.cu).
 struct PrepConv {  // fp32 rows x cols (lds) -> fp16 hi [lo] (ldd), triangle mode tri (convert_f32_f16)
   long long rows = 0, cols = 0;
   const float* src = nullptr;
