@@ -42,9 +42,8 @@
 // `kchunk` K-blocks the epilogue adds acc0 to FP32 registers with
 // round-to-nearest adds: the tensor core's own FP32 accumulation truncates,
 // which would cost ~K/16 ulps. The correction, 2^-11 of the result, stays in
-// its accumulator over the tile's whole K range and is added once: its
-// truncation is 2^-11 of the main accumulator's, and the fold reads half the
-// TMEM columns and rounds half as often.
+// its accumulator for kCorrRounds such folds, so that most of them read half
+// the TMEM columns and round half as often.
 #pragma once
 #include "tb_ptx.cuh"
 
@@ -110,6 +109,20 @@ __device__ __forceinline__ int static_next(const GemmArgs& a, int b, int nb, int
 // the MMA issuer, the four epilogue warps and (prefetch variants) the C
 // loader each take the indices in order and release the slot.
 constexpr int kTileQ = 4;
+
+// Split mode: main folds for which the correction stays in its accumulator (a
+// stretch; 128 K-blocks, K = 8192, with the default fold interval). The sum in
+// TMEM truncates about twice per 16-deep step, so a stretch loses at most
+// 2^-22 * 512 / 2 = 6e-5 of a correction that is at most 2^-11 of the sum of
+// the products' magnitudes: half an FP32 unit roundoff of that sum, whatever
+// K is. Over the whole K range the loss grows with K: with lo parts of one
+// sign the correction was off by 1.1e-4 at K = 16384, 2.1e-4 at 32768 and
+// 8.6e-4 at 131072, now 5e-5 at each. Each stretch end adds one rounding per
+// element; folded every 16 rounds or every 8 the error of U[-1, 1] operands
+// at K = 16384 rose from 3.72e-7 to 3.73e-7 or 3.76e-7, and folding every
+// round (two roundings a fold) made it 3.98e-7. Time: within the runs' spread
+// (SGEMM 4096 x 4096 x 32768 on pairs 2.62 to 2.69 ms before and after).
+constexpr int kCorrRounds = 32;
 
 // The next tile of a consumer role: static striding, or the producer's
 // queue (q/ph: the role's ring position). EPI: called by the 128 threads of
@@ -191,7 +204,7 @@ struct GemmCfg {
   static constexpr int STAGE_BYTES = NOPS * (A_BYTES + B_BYTES);
   static constexpr int STAGES = BN == 64 ? (SPLIT ? 4 : 6) : FP8 ? 6 : PF ? (SPLIT ? 3 : 4) : (SPLIT ? 3 : (BN == 128 ? 6 : 4));
   // TMEM: two main accumulators (alternating by round), then two corrections
-  // (alternating by tile)
+  // (alternating by stretch)
   static constexpr int CORR_COL = 2 * BN;
   static constexpr int TMEM_COLS = (SPLIT ? 4 : 2) * BN;
   static_assert(TMEM_COLS <= 512, "TMEM budget");
@@ -667,6 +680,7 @@ struct TileAcc {
           release(&tempty[buf]);
         }
       } else {
+        int left = kCorrRounds;  // rounds up to the end of the correction's stretch
         for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk) {
           if (!round()) return false;
           const uint32_t ta = tmem + (uint32_t)(buf * Cfg::BN);
@@ -675,8 +689,17 @@ struct TileAcc {
             for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
           });
           release(&tempty[buf]);
+          if (--left == 0 && tile.w - c0k > args.kchunk) {  // the round's commit covers the correction's MMAs
+            tmem_for32<Cfg::GC>(tmem + (uint32_t)(Cfg::CORR_COL + (nt & 1) * Cfg::BN), [&](int c0, const float* w) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(args.corr_scale, w[j], acc[c0 + j]);
+            });
+            release(&xempty[nt & 1]);
+            ++nt;
+            left = kCorrRounds;
+          }
         }
-        if (tile.z < tile.w) {  // the last round's commit covers the correction's MMAs
+        if (tile.z < tile.w) {  // the correction of the last stretch
           const uint32_t tc = tmem + (uint32_t)(Cfg::CORR_COL + (nt & 1) * Cfg::BN);
 #pragma unroll
           for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
@@ -858,12 +881,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
     // Main accumulation in rounds, one TMEM buffer each: plain mode runs a
     // tile's whole K range in one round; split mode closes a round every
     // `kchunk` K-blocks and FP8 every K-block. Split mode's correction
-    // products go to the tile's own accumulator over all its rounds.
+    // products go to an accumulator of their own for kCorrRounds rounds.
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 0;
       int it = 0;  // round counter (selects the main buffer and its phase)
-      int nt = 0;  // tile counter (selects the correction buffer and its phase)
+      int nt = 0;  // stretch counter (selects the correction buffer and its phase)
       bool ok = true;
       bool any = false;
       const int kc = Cfg::FOLD ? args.kchunk : (1 << 30);
@@ -873,16 +896,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
            t >= 0 && ok;
            t = next_tile<false>(args, t, tq_idx, tq_full, tq_empty, tq, tq_ph, abort_flag, kDevErrTimeoutMma)) {
         const int4 tile = args.tiles[t];
-        const uint32_t x0 = tmem_base + (uint32_t)(Cfg::CORR_COL + (nt & 1) * BN);
-        if (Cfg::SPLIT && tile.z < tile.w) {
-          if (!mbar_wait(&xempty[nt & 1], ((uint32_t)(nt >> 1) & 1u) ^ 1u, abort_flag, args.err, kDevErrTimeoutMma)) {
-            ok = false;
-            break;
-          }
-          ++nt;
-        }
+        uint32_t x0 = 0;
+        int xkb = 0, left = 0;  // the correction's stretch: first K-block, rounds left
         for (int c0 = tile.z; c0 < tile.w && ok; c0 += kc, ++it) {
           const int c1 = (tile.w - c0 > kc) ? c0 + kc : tile.w;
+          if (Cfg::SPLIT && --left < 0) {
+            if (!mbar_wait(&xempty[nt & 1], ((uint32_t)(nt >> 1) & 1u) ^ 1u, abort_flag, args.err,
+                           kDevErrTimeoutMma)) {
+              ok = false;
+              break;
+            }
+            x0 = tmem_base + (uint32_t)(Cfg::CORR_COL + (nt & 1) * BN);
+            xkb = c0;
+            left = kCorrRounds - 1;
+            ++nt;
+          }
           const int buf = it & 1;
           const uint32_t tph = (uint32_t)(it >> 1) & 1u;
           if (!mbar_wait(&tempty[buf], tph ^ 1u, abort_flag, args.err, kDevErrTimeoutMma)) {
@@ -911,7 +939,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
               if constexpr (Cfg::SPLIT) {
                 const uint64_t da_lo = operand_desc<Cfg::A_MN>(a_hi + Cfg::A_BYTES, kk);
                 const uint64_t db_lo = operand_desc<Cfg::B_MN>(b_hi + Cfg::B_BYTES, kk);
-                umma_f16(x0, da, db_lo, Cfg::IDESC, (kb > tile.z || kk > 0) ? 1u : 0u);
+                umma_f16(x0, da, db_lo, Cfg::IDESC, (kb > xkb || kk > 0) ? 1u : 0u);
                 umma_f16(x0, da_lo, db, Cfg::IDESC, 1u);
               }
             }
@@ -1015,7 +1043,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
 // MMAs: while a round's last correction MMAs run (1024 cycles per SM), the
 // epilogue reads the main accumulator, and the next round's main MMAs find it
 // free. Buffer 0 is the main accumulator (one phase a round), buffer 1 the
-// correction (one phase a tile). Per 64-deep K block and SM the 256 x 256 tile
+// correction (one phase a stretch of kCorrRounds). Per 64-deep K block and SM the 256 x 256 tile
 // moves 64 KB into shared memory and 96 KB out of it for 1536 MMA cycles,
 // where 256 x 128 tiles (which left room to double-buffer) moved 96 + 144 KB.
 // The tensor pipe is 93 % busy while the SM is active against 65 %: SYR2K n = 16384, k = 4096 went from 6.0
@@ -1118,6 +1146,7 @@ struct PairAcc {
           release(b);
         }
       } else {
+        int left = kCorrRounds;  // rounds up to the end of the correction's stretch
         for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk, ++it) {
           if (!wait(0, (uint32_t)it & 1u)) return false;
           tmem_for32<Cfg::GC>(tmem, [&](int c0, const float* v) {
@@ -1125,18 +1154,16 @@ struct PairAcc {
             for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
           });
           release(0);
-        }
-        if (tile.z < tile.w) {
-          if (!wait(1, (uint32_t)nt & 1u)) return false;
-          ++nt;
+          if (--left == 0 || tile.w - c0k <= args.kchunk) {
+            if (!wait(1, (uint32_t)nt & 1u)) return false;
+            tmem_for32<Cfg::GC>(tmem + Cfg::BN, [&](int c0, const float* w) {
 #pragma unroll
-          for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
-            float w[32];
-            tmem_ld32(tmem + Cfg::BN + c0, w);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(args.corr_scale, w[j], acc[c0 + j]);
+              for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(args.corr_scale, w[j], acc[c0 + j]);
+            });
+            release(1);
+            ++nt;
+            left = kCorrRounds;
           }
-          release(1);
         }
       }
       return true;
@@ -1275,11 +1302,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       if (leader && lane == 0) {
         int s = 0;
         uint32_t ph = 0;
-        int it = 0, nt = 0;  // rounds and (split) tiles: buffers and phases, as in gemm_kernel
+        int it = 0, nt = 0;  // rounds and (split) stretches: buffers and phases, as in gemm_kernel
         bool ok = true, any = false;
         const int kc = Cfg::FOLD ? args.kchunk : (1 << 30);
         for (int t = static_first(args, pair); t >= 0 && ok; t = static_next(args, pair, npairs, t)) {
           const int4 tile = args.tiles[t];
+          int xkb = tile.z, left = kCorrRounds;  // split: the correction's stretch, as in gemm_kernel
           for (int c0 = tile.z; c0 < tile.w && ok; c0 += kc, ++it) {
             const int c1 = (tile.w - c0 > kc) ? c0 + kc : tile.w;
             const int buf = Cfg::SPLIT ? 0 : (it & 1);
@@ -1309,7 +1337,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
               any = true;
               if constexpr (Cfg::SPLIT) {
                 if (kb == c1 - 1) tc_commit_pair(&tfull[0], 3);  // the round's main products are issued
-                if (kb == tile.z) {
+                if (kb == xkb) {
                   if (!mbar_wait(&tempty[1], ((uint32_t)nt & 1u) ^ 1u, abort_flag, args.err, kDevErrTimeoutMma)) {
                     ok = false;
                     break;
@@ -1320,7 +1348,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
                 for (int kk = 0; kk < 4; ++kk) {
                   const uint64_t da = operand_desc<Cfg::A_MN>(a, kk), db = operand_desc<Cfg::B_MN>(b, kk);
                   umma_f16_pair(d0 + BN, da, operand_desc<Cfg::B_MN>(b + Cfg::B_BYTES, kk), Cfg::IDESC,
-                                (kb > tile.z || kk > 0) ? 1u : 0u);
+                                (kb > xkb || kk > 0) ? 1u : 0u);
                   umma_f16_pair(d0 + BN, operand_desc<Cfg::A_MN>(a + Cfg::A_BYTES, kk), db, Cfg::IDESC, 1u);
                 }
               }
@@ -1331,13 +1359,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
               }
             }
             if (!ok) break;
-            if constexpr (!Cfg::SPLIT) tc_commit_pair(&tfull[buf], 3);
-          }
-          if (!ok) break;
-          if constexpr (Cfg::SPLIT) {
-            if (tile.z < tile.w) {
-              tc_commit_pair(&tfull[1], 3);
-              ++nt;
+            if constexpr (Cfg::SPLIT) {
+              if (--left == 0 || c1 == tile.w) {
+                tc_commit_pair(&tfull[1], 3);  // the stretch's correction products are issued
+                ++nt;
+                xkb = c1;
+                left = kCorrRounds;
+              }
+            } else {
+              tc_commit_pair(&tfull[buf], 3);
             }
           }
         }

@@ -366,12 +366,18 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
         const DagTask task = args.tasks[t];
         const bool split = task.meta.y != 0;
         const int kc = split ? args.kchunk : (1 << 30);
-        // split tasks: the correction stays in the upper half of the first
-        // round's buffer over all rounds (later rounds use lower halves only)
-        const uint32_t x0 = tmem_base + (uint32_t)((it & 1) * 256 + 128);
+        // split tasks: the correction stays in the upper half of its stretch's
+        // first round's buffer (the later rounds use lower halves only)
+        uint32_t x0 = 0;
+        int xkb = 0, left = 0;  // the stretch's first K-block, rounds left
         for (int c0 = task.tile.z; c0 < task.tile.w && ok; c0 += kc, ++it) {
           const int c1 = (task.tile.w - c0 > kc) ? c0 + kc : task.tile.w;
           const int buf = it & 1;
+          if (--left < 0) {
+            x0 = tmem_base + (uint32_t)(buf * 256 + 128);
+            xkb = c0;
+            left = kCorrRounds - 1;
+          }
           const uint32_t tph = (uint32_t)(it >> 1) & 1u;
           if (!mbar_wait(&tempty[buf], tph ^ 1u, abort_flag, args.err, kDevErrTimeoutMma)) {
             ok = false;
@@ -407,7 +413,7 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
                 const uint64_t da_lo = operand_desc<A_MN>(st + kDagABytes, kk);
                 const uint64_t db_lo = operand_desc<B_MN>(st_lo, kk);
                 umma_f16(d0, da, db, IDESC_SPLIT, acc);
-                umma_f16(x0, da, db_lo, IDESC_SPLIT, (kb > task.tile.z || kk > 0) ? 1u : 0u);
+                umma_f16(x0, da, db_lo, IDESC_SPLIT, (kb > xkb || kk > 0) ? 1u : 0u);
                 umma_f16(x0, da_lo, db, IDESC_SPLIT, 1u);
               } else {
                 umma_f16(d0, da, operand_desc<B_MN>(st + kDagABytes, kk), IDESC_PLAIN, acc);
@@ -510,11 +516,12 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
         float acc[128];
 #pragma unroll
         for (int j = 0; j < 128; ++j) acc[j] = 0.f;
-        // main sums every round; the correction (upper half of the first
-        // round's buffer) once at the end. The buffers of the last two rounds
-        // go back together after that: one of them holds the correction.
-        const uint32_t xacc = tmem_base + lane_addr + (uint32_t)((it & 1) * 256 + 128);
-        int held = -1;
+        // main sums every round; the correction (upper half of its stretch's
+        // first round's buffer) at the stretch's end. The buffers of a
+        // stretch's last two rounds go back together after that: one of them
+        // holds the correction.
+        uint32_t xacc = 0;
+        int held = -1, rounds = 0;  // rounds of the stretch still to come
         auto give_back = [&](int b) {
           tc_fence_before();
           __syncwarp();
@@ -522,6 +529,10 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
         };
         for (int c0k = task.tile.z; c0k < task.tile.w; c0k += args.kchunk) {
           const int buf = it & 1;
+          if (rounds == 0) {
+            xacc = tmem_base + lane_addr + (uint32_t)(buf * 256 + 128);
+            rounds = min(kCorrRounds, (task.tile.w - c0k + args.kchunk - 1) / args.kchunk);
+          }
           const uint32_t tph = (uint32_t)(it >> 1) & 1u;
           ++it;
           if (named_bar_any(1, 128, !mbar_wait(&tfull[buf], tph, abort_flag, args.err, kDevErrTimeoutEpilogue))) {
@@ -537,8 +548,7 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
 #pragma unroll
             for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
           }
-          const int left = task.tile.w - c0k;  // K-blocks from this round on
-          if (left <= args.kchunk) {           // the last round: every product is in
+          if (--rounds == 0) {  // the stretch's last round: its products are in
 #pragma unroll
             for (int c0 = 0; c0 < 128; c0 += 32) {
               float w[32];
@@ -547,8 +557,9 @@ __global__ void __launch_bounds__(kDagThreads, 1) trsm_dag_kernel(const __grid_c
               for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(P.corr_scale, w[j], acc[c0 + j]);
             }
             if (held >= 0) give_back(held);
+            held = -1;
             give_back(buf);
-          } else if (left <= 2 * args.kchunk) {
+          } else if (rounds == 1) {
             held = buf;
           } else {
             give_back(buf);
