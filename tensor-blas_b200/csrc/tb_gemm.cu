@@ -461,12 +461,15 @@ tb_status gemm_launch_plan(GemmCall& c, const std::vector<int4>& plan, cudaStrea
   std::vector<int4> merged;
   if (c.pair) {
     merged = merge_pairs(plan, c.M, c.N);
-    // split: a 256 x 256 pair tile takes about 1.45 times a 128 x 128 single
-    // CTA's time (four times the work at a better rate on two SMs), so the
-    // pairs lose where they leave more of the last wave empty
+    // split and FP8: a 256 x 256 pair tile takes about 1.45 times a 128 x 128
+    // single CTA's time (four times the work at a better rate on two SMs), so
+    // the pairs lose where they leave more of the last wave empty. FP8 on a
+    // B200, waves of singles / pairs and their times in us: 1024^3 1 / 1, 16 /
+    // 21; 1024 x 1024 x 8192 1 / 1, 47 / 55; 1100 x 8192 x 2048 4 / 3, 59 /
+    // 61; 2304^3 3 / 2, 49 / 45; 2048^3 2 / 1, 35 / 27; 4096^3 7 / 4, 158 / 121
     const long sms = sm_count(), ws = ((long)plan.size() + sms - 1) / sms,
                wp = ((long)merged.size() + sms / 2 - 1) / (sms / 2);
-    if (!c.fp8 && c.split == Split::kHiLo && wp * 1.45 > (double)ws) c.pair = false;
+    if ((c.fp8 || c.split == Split::kHiLo) && wp * 1.45 > (double)ws) c.pair = false;
   }
   if (c.pair) {
     TB_TRY(set_tiles(c, merged, std::min<int>((int)merged.size(), sm_count() / 2), stream));
