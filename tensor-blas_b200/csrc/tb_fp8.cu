@@ -47,6 +47,16 @@ __device__ __forceinline__ float q8_load(const Q8Src& s, long long i, long long 
   }
 }
 
+// The scale of blocks that the mask zeroes wholly: the epilogue skips their
+// products. A pair tile's K range spans its four 128 x 128 parts, so such a
+// block of the triangle also meets blocks of the other operand that its own
+// rows or columns do not reach, and zero times an infinity there is NaN.
+constexpr float kMaskedScale = -1.f;
+
+__device__ __forceinline__ bool q8_masked(const Q8Src& s, long long r0, long long p0) {
+  return s.mask == 1 ? p0 > r0 + kQB - 1 : (s.mask == 2 && p0 + kQB - 1 < r0);
+}
+
 // How a 128 x 128 block at (r0, p0) can be read: 0 / 1 as a plain kind-0 /
 // kind-1 block (every element inside the operand and unmasked, 16-byte
 // aligned rows), 2 when the mask zeroes all of it, -1 otherwise (diagonal,
@@ -54,13 +64,9 @@ __device__ __forceinline__ float q8_load(const Q8Src& s, long long i, long long 
 __device__ __forceinline__ int q8_block_kind(const Q8Src& s, long long r0, long long p0, long long rows,
                                              long long K, bool vec) {
   if (!vec || r0 + kQB > rows || p0 + kQB > K) return -1;
-  if (s.mask == 1) {  // keeps p <= i
-    if (p0 > r0 + kQB - 1) return 2;
-    if (p0 + kQB - 1 > r0) return -1;
-  } else if (s.mask == 2) {  // keeps p >= i
-    if (p0 + kQB - 1 < r0) return 2;
-    if (p0 < r0 + kQB - 1) return -1;
-  }
+  if (q8_masked(s, r0, p0)) return 2;
+  if (s.mask == 1 && p0 + kQB - 1 > r0) return -1;  // keeps p <= i
+  if (s.mask == 2 && p0 < r0 + kQB - 1) return -1;  // keeps p >= i
   if (s.unit && r0 < p0 + kQB && p0 < r0 + kQB) return -1;
   switch (s.kind) {
     case 0:
@@ -111,7 +117,7 @@ __global__ void __launch_bounds__(256) q8_kernel(Q8Src src, long long rows, long
   float* const sc = scales + (long long)blockIdx.x * scale_ld + kb_off + blockIdx.y;
   const int kind = q8_block_kind(src, r0, p0, rows, K, vec != 0);
   if (kind == 2) {
-    if (t == 0) *sc = 1.f;
+    if (t == 0) *sc = kMaskedScale;
     for (int job = t; job < kQB * (kQB / 16); job += 256) {
       const int r = job >> 3, c = (job & 7) * 16;
       *reinterpret_cast<uint4*>(Q + (r0 + r) * ldq + qoff + p0 + c) = make_uint4(0, 0, 0, 0);
@@ -128,7 +134,7 @@ __global__ void __launch_bounds__(256) q8_kernel(Q8Src src, long long rows, long
     }
     const float m = q8_block_max(amax, red);
     const float scale = m > 0.f ? m / 448.f : 1.f;
-    if (t == 0) *sc = scale;
+    if (t == 0) *sc = q8_masked(src, r0, p0) ? kMaskedScale : scale;
     for (int job = t; job < kQB * (kQB / 16); job += 256) {
       const int r = job >> 3, c = (job & 7) * 16;
       const long long gi = r0 + r;

@@ -423,9 +423,10 @@ static tb_status set_tiles(GemmCall& c, const std::vector<int4>& tiles, int work
 }
 
 // Vertically and horizontally adjacent tiles of a plan merged into 256 x 256
-// pair tiles (the K range of a pair tile spans its parts; products outside an
+// pair tiles. The K range of a pair tile spans its parts'; products outside an
 // operand's support multiply stored zeros, and masked outputs are never
-// written).
+// written. An infinity or NaN that meets such a zero reaches the whole tile
+// (FP8 skips those blocks).
 static std::vector<int4> merge_pairs(const std::vector<int4>& plan, int M, int N) {
   // a flat index over 256 x 256 blocks: plans have thousands of tiles and
   // this runs on every call

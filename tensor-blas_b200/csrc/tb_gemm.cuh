@@ -1139,10 +1139,11 @@ struct PairAcc {
           const int b = it & 1;
           if (!wait(b, (uint32_t)(it >> 1) & 1u)) return false;
           const uint32_t ta = tmem + (uint32_t)(b * Cfg::BN);
-          tmem_for32<Cfg::GC>(ta, [&](int c0, const float* v) {
+          if (!(s < 0.f))  // negative: a block outside a triangle, all zeros
+            tmem_for32<Cfg::GC>(ta, [&](int c0, const float* v) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(s, v[j], acc[c0 + j]);
-          });
+              for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(s, v[j], acc[c0 + j]);
+            });
           release(b);
         }
       } else {
