@@ -1,7 +1,8 @@
-"""256 x 256 CTA-pair tiles of the FP8 form against the single-CTA 128 x 128
-tiles (TB_GEMM_PAIR=0), at sizes that the dispatch sends to pairs: the
-library's launch counters show which kernel ran, the results must be
-bit-identical and agree with FP64. A launch takes pairs when its waves of pair
+"""256 x 256 CTA-pair tiles of the split and FP8 forms against the single-CTA
+128 x 128 tiles (TB_GEMM_PAIR=0, for split also TB_GEMM_PAIR_SPLIT=0), at sizes
+that the dispatch sends to pairs: the library's launch counters show which
+kernel ran, the results must be bit-identical (but for the split upper TRMM,
+whose pair tiles fold at other K blocks) and agree with FP64. A launch takes pairs when its waves of pair
 tiles, 1.45 single-tile times each, are fewer than those of single tiles; on
 either side of that line the counters must show it. The engine is read once
 per process, so each setting runs in its own subprocess."""
@@ -14,8 +15,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-FP8 = 2
-BOUND = {FP8: 8e-2}
+SPLIT, FP8 = 1, 2
+BOUND = {SPLIT: 2e-6, FP8: 8e-2}
 
 SCRIPT = r"""
 import ctypes, hashlib, sys, numpy as np, torch
@@ -75,15 +76,15 @@ for case in eval(sys.argv[2]):
 """
 
 
-def _run(pair, cases):
+def _run(pair, cases, switch="TB_GEMM_PAIR"):
     out = subprocess.run([sys.executable, "-c", SCRIPT, os.path.join(ROOT, "tensor-blas_b200", "python"), repr(cases)],
-                         env=dict(os.environ, TB_GEMM_PAIR=pair), capture_output=True, text=True, timeout=900)
+                         env=dict(os.environ, **{switch: pair}), capture_output=True, text=True, timeout=900)
     assert out.returncode == 0, out.stderr[-2000:]
     return [(d, int(p), float(e)) for d, p, e in (line.split() for line in out.stdout.splitlines())]
 
 
-def _check_pairs(cases):
-    for case, pair, single in zip(cases, _run("1", cases), _run("0", cases)):
+def _check_pairs(cases, switch="TB_GEMM_PAIR"):
+    for case, pair, single in zip(cases, _run("1", cases, switch), _run("0", cases, switch)):
         print(case, pair, single)
         assert pair[1] == 1 and single[1] == 0, case  # the two engines ran
         assert pair[2] <= BOUND[case[4]] and single[2] <= BOUND[case[4]], case
@@ -96,6 +97,18 @@ def test_fp8_pair_tiles_match_single_cta_tiles():
              ("symm", 2100, 1700, 0, FP8, 0.5), ("trmm", 2050, 1930, 0, FP8, 0.0), ("trmm_u", 1999, 2301, 0, FP8, 0.0),
              ("gemmTN", 2000, 2100, 129, FP8, 0.5)]
     assert all(same for _, same in _check_pairs(cases))
+
+
+@pytest.mark.parametrize("switch", ["TB_GEMM_PAIR", "TB_GEMM_PAIR_SPLIT"])
+def test_split_pair_tiles_match_single_cta_tiles(switch):
+    cases = [("syrk", 0, 2304, 2048, SPLIT, 0.0), ("syrk", 0, 2500, 1100, SPLIT, 0.5),
+             ("syrkT", 0, 2432, 1536, SPLIT, 0.0), ("syr2k", 0, 2304, 1025, SPLIT, 0.0),
+             ("trmm", 2048, 2048, 0, SPLIT, 0.0), ("trmm_u", 2048, 1990, 0, SPLIT, 0.0),
+             ("symm", 2048, 2048, 0, SPLIT, 0.5), ("gemmNN", 2048, 2048, 1536, SPLIT, 0.0),
+             ("gemmTN", 1990, 2048, 1100, SPLIT, 0.5), ("gemmNT", 2048, 1801, 1537, SPLIT, 0.0),
+             ("gemmTT", 2002, 2001, 1100, SPLIT, 0.5)]
+    differ = [case for case, same in _check_pairs(cases, switch) if not same]
+    assert [case[0] for case in differ] in ([], ["trmm_u"]), differ
 
 
 def test_fp8_engine_follows_the_waves():
