@@ -328,10 +328,9 @@ tb_status gemm_launch(GemmCall& c, cudaStream_t stream) {
   const bool pf = c.kblocks > 0 && c.kblocks <= kGemmPfMaxKb;
   const int bn = c.bn ? c.bn : gemm_bn(c.split, c.kblocks);
   if (bn == 64) {
-    if (split) TB_BY_LAYOUT(TB_SINGLE, 64, 3, true);
-    TB_BY_LAYOUT(TB_SINGLE, 64, 1, true);
+    if (split) TB_BY_LAYOUT(TB_SINGLE, 64, 3, false);
+    TB_BY_LAYOUT(TB_SINGLE, 64, 1, false);
   }
-  if (split && pf) TB_BY_LAYOUT(TB_SINGLE, 128, 3, true);
   if (split) TB_BY_LAYOUT(TB_SINGLE, 128, 3, false);
   if (pf) TB_BY_LAYOUT(TB_SINGLE, 128, 1, true);
   if (bn == 128) TB_BY_LAYOUT(TB_SINGLE, 128, 1, false);

@@ -180,8 +180,9 @@ constexpr int kGemmThreads = 32 * (kEpiWarp0 + 4 * kEpiGroups);
 
 // Shared memory left beside the operand stages goes to the C slots: a group's
 // loader ring runs that many 8 KB chunks ahead of its epilogue.
-// PF variants serve launches whose tiles have few K-blocks: there C, not the
-// MMA, bounds the tile, so they trade operand stages for C slots.
+// PF variants (plain, 128 x 128) serve launches whose tiles have few K-blocks:
+// there C, not the MMA, bounds the tile, so they trade operand stages for C
+// slots. A split tile's three stages leave room for two slots a group at any K.
 // FP8 variant: e4m3 K-major operands scaled per 128 x 128 block; the
 // accumulator is folded into fp32 registers after every 128-deep K block
 // with the product of the two blocks' scales.
@@ -191,6 +192,7 @@ template <int BN_, int NSPLIT_, bool A_MN_, bool B_MN_, bool PF_ = false, bool F
 struct GemmCfg {
   static constexpr bool PF = PF_;
   static constexpr bool FP8 = FP8_;
+  static_assert(!PF || (BN_ == 128 && NSPLIT_ == 1 && !FP8), "PF: plain 128 x 128 tiles");
   static constexpr int ELEM = FP8 ? 1 : 2;       // operand bytes per element
   static constexpr int BM = 128, BN = BN_, BK = 128 / ELEM;  // one 128-byte swizzle row of K per stage
   static constexpr int KSTEPS = 4;               // MMAs per stage (K = 16 fp16 / 32 fp8 each)
@@ -202,7 +204,7 @@ struct GemmCfg {
   static constexpr int A_BYTES = BM * BK * ELEM;
   static constexpr int B_BYTES = BN * BK * ELEM;
   static constexpr int STAGE_BYTES = NOPS * (A_BYTES + B_BYTES);
-  static constexpr int STAGES = BN == 64 ? (SPLIT ? 4 : 6) : FP8 ? 6 : PF ? (SPLIT ? 3 : 4) : (SPLIT ? 3 : (BN == 128 ? 6 : 4));
+  static constexpr int STAGES = SPLIT ? (BN == 64 ? 4 : 3) : (PF || BN == 256) ? 4 : 6;
   // TMEM: two main accumulators (alternating by round), then two corrections
   // (alternating by stretch)
   static constexpr int CORR_COL = 2 * BN;
@@ -210,7 +212,7 @@ struct GemmCfg {
   static_assert(TMEM_COLS <= 512, "TMEM budget");
   static constexpr int GC = BN / kEpiGroups;              // columns of one epilogue group
   static constexpr int CHUNK_BYTES = 128 * kEpiCols * 4;  // one staged 128 x 16 fp32 chunk
-  static constexpr int C_SLOTS = BN == 64 || (PF && SPLIT) ? 2 : PF ? 6 : 2;  // per group (BN = 64: all its chunks)
+  static constexpr int C_SLOTS = PF ? 6 : 2;              // per group (BN = 64: all its chunks)
   static constexpr int GROUP_BYTES = C_SLOTS * CHUNK_BYTES;
   static constexpr int EPI_BYTES = kEpiGroups * GROUP_BYTES;
   static constexpr int BAR_BYTES = 512;
