@@ -682,26 +682,19 @@ struct TileAcc {
           release(&tempty[buf]);
         }
       } else {
-        int left = kCorrRounds;  // rounds up to the end of the correction's stretch
-        for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk) {
+        // one round's main sums
+        auto fold_round = [&]() {
           if (!round()) return false;
-          const uint32_t ta = tmem + (uint32_t)(buf * Cfg::BN);
-          tmem_for32<Cfg::GC>(ta, [&](int c0, const float* v) {
+          tmem_for32<Cfg::GC>(tmem + (uint32_t)(buf * Cfg::BN), [&](int c0, const float* v) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) acc[c0 + j] += v[j];
           });
           release(&tempty[buf]);
-          if (--left == 0 && tile.w - c0k > args.kchunk) {  // the round's commit covers the correction's MMAs
-            tmem_for32<Cfg::GC>(tmem + (uint32_t)(Cfg::CORR_COL + (nt & 1) * Cfg::BN), [&](int c0, const float* w) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(args.corr_scale, w[j], acc[c0 + j]);
-            });
-            release(&xempty[nt & 1]);
-            ++nt;
-            left = kCorrRounds;
-          }
-        }
-        if (tile.z < tile.w) {  // the correction of the last stretch
+          return true;
+        };
+        // the correction (the last round's commit covers its MMAs) with the
+        // main sums, in its place
+        auto fold_stretch = [&]() {
           const uint32_t tc = tmem + (uint32_t)(Cfg::CORR_COL + (nt & 1) * Cfg::BN);
 #pragma unroll
           for (int c0 = 0; c0 < Cfg::GC; c0 += 32) {
@@ -709,11 +702,42 @@ struct TileAcc {
             tmem_ld32(tc + c0, w);
 #pragma unroll
             for (int j = 0; j < 32; ++j) w[j] = fmaf(args.corr_scale, w[j], acc[c0 + j]);
-            // the folded tile takes the place of the correction it was folded with
             tmem_st32(tc + c0, w);
           }
           tmem_st_wait();
           folded = tc;
+        };
+        // Stretches before the last. On 64-column tiles, whose short launches
+        // are bound by fetching their code, the same fold serves them and its
+        // sums are read back (TRSM 4096 x 256 0.5 to 2 % faster than with a
+        // copy of it); the wider tiles' registers do not allow that.
+        if constexpr (Cfg::GC == 32) {
+          for (int c0k = tile.z; c0k < tile.w;) {
+            const int cend = min(tile.w, c0k + kCorrRounds * args.kchunk);
+            for (; c0k < cend; c0k += args.kchunk)
+              if (!fold_round()) return false;
+            fold_stretch();
+            if (c0k < tile.w) {
+              tmem_ld32(folded, acc);
+              release(&xempty[nt & 1]);
+              ++nt;
+            }
+          }
+        } else {
+          int left = kCorrRounds;
+          for (int c0k = tile.z; c0k < tile.w; c0k += args.kchunk) {
+            if (!fold_round()) return false;
+            if (--left == 0 && tile.w - c0k > args.kchunk) {
+              tmem_for32<Cfg::GC>(tmem + (uint32_t)(Cfg::CORR_COL + (nt & 1) * Cfg::BN), [&](int c0, const float* w) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) acc[c0 + j] = fmaf(args.corr_scale, w[j], acc[c0 + j]);
+              });
+              release(&xempty[nt & 1]);
+              ++nt;
+              left = kCorrRounds;
+            }
+          }
+          if (tile.z < tile.w) fold_stretch();
         }
       }
       return true;
