@@ -366,7 +366,6 @@ extern "C" tb_status tb_batch_create(tb_batch_t* out, int count, const int* kind
   const int nprob = (int)probs.size();
   std::vector<GemmArgs> hargs(nprob);
   for (int i = 0; i < nprob; ++i) {
-    probs[i].epi_cols = kEpiCols;
     tb_status st = gemm_build_args(probs[i], &hargs[i]);
     if (st != TB_SUCCESS) {
       tb_batch_destroy(b);

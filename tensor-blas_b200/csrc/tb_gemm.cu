@@ -296,10 +296,9 @@ static double gemm_algorithmic_bytes(const GemmCall& c) {
   return ops + cbytes + side;
 }
 
-tb_status gemm_launch(GemmCall& c, cudaStream_t stream) {
+tb_status gemm_launch(const GemmCall& c, cudaStream_t stream) {
   if (c.num_tiles <= 0) return TB_SUCCESS;
   GemmArgs a;
-  c.epi_cols = kEpiCols;
   TB_TRY(gemm_build_args(c, &a));
   const double bytes = gemm_algorithmic_bytes(c);
   const bool split = c.split == Split::kHiLo;

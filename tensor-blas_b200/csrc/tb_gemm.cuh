@@ -45,6 +45,7 @@
 // its accumulator for kCorrRounds such folds, so that most of them read half
 // the TMEM columns and round half as often.
 #pragma once
+#include "tb_internal.h"
 #include "tb_ptx.cuh"
 
 namespace tb {
@@ -174,7 +175,6 @@ __device__ __forceinline__ const GemmArgs& tile_problem(const GemmArgs& args, in
 // product of 6003 x 512 with an odd leading dimension went from 73 to 30 us,
 // the 512-instance batch from 6.5 to 5.1 ms.
 constexpr int kEpiGroups = 2;
-constexpr int kEpiCols = 16;
 constexpr int kEpiWarp0 = 4;  // first epilogue warp
 constexpr int kGemmThreads = 32 * (kEpiWarp0 + 4 * kEpiGroups);
 

@@ -96,6 +96,9 @@ enum class Split { kPlain = 1, kHiLo = 3 };
 // environment (read once).
 int split_kchunk();
 
+// Columns of a C chunk of the GEMM engine's epilogue (one TMA box).
+constexpr int kEpiCols = 16;
+
 struct GemmCall {
   Operand a_hi, a_lo, b_hi, b_lo;  // lo used in kHiLo only
   Split split = Split::kPlain;
@@ -121,7 +124,7 @@ struct GemmCall {
   // scale_ld K blocks per row block); tiles 128 x 128.
   bool pair = false;  // set by gemm_launch_plan: 256 x 256 tiles on CTA pairs (cta_group::2)
   int bn = 0;         // set by gemm_launch_plan: tile width of a single-CTA launch (0: gemm_bn(split, kblocks))
-  int epi_cols = 32;  // columns of the TMA boxes the epilogue moves C and the side copies in
+  int epi_cols = kEpiCols;  // columns of the TMA boxes C moves in (the persistent TRSM's kernel: 32)
   bool fp8 = false;
   const float* scale_a = nullptr;
   const float* scale_b = nullptr;
@@ -140,7 +143,7 @@ constexpr int kGemmBNFp8 = 128;  // FP8 tiles: 128 x 128, K blocks of 128
 int gemm_bn(Split s);
 int gemm_bn(Split s, int kblocks);
 
-tb_status gemm_launch(GemmCall& call, cudaStream_t stream);
+tb_status gemm_launch(const GemmCall& call, cudaStream_t stream);
 // Whether kernels that wait in grid_dep_wait may be launched with programmatic
 // stream serialization on this stream.
 bool dependent_launch(cudaStream_t stream);

@@ -188,7 +188,6 @@ tb_status syrk_splitk(long n, long k, float alpha, float beta, float* C, long ld
     c.beta = 0.f;
     c.tri = upper ? 2 : 1;
     c.diag = 0;
-    c.epi_cols = kEpiCols;
     TB_TRY(gemm_build_args(c, &probs[q]));
     const std::vector<int4> part = upper ? plan_upper((int)n, 256, k0, k1) : plan_lower((int)n, 256, k0, k1);
     tiles.insert(tiles.end(), part.begin(), part.end());

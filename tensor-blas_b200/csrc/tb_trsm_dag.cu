@@ -1055,6 +1055,7 @@ tb_status trsm_solve_dag(TrsmCtx& c, const std::vector<long>& leaf_start, float*
   std::vector<GemmArgs> hops(ops.size());
   double flops = 0;
   for (size_t i = 0; i < ops.size(); ++i) {
+    ops[i].call.epi_cols = 32;  // dag_chunk's boxes
     TB_TRY(gemm_build_args(ops[i].call, &hops[i]));
     flops += ops[i].call.flops;
   }
