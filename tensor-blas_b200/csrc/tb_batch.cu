@@ -471,7 +471,6 @@ extern "C" tb_status tb_batch_create(tb_batch_t* out, int count, const int* kind
   device_error_word();
   sm_count();
   TB_TRY(gemm_prepare_grouped());
-  TB_TRY(trsm_prepare_grouped());
   *out = b;
   return TB_SUCCESS;
 }

@@ -319,7 +319,6 @@ tb_status trsm_solve_dag(TrsmCtx& c, const std::vector<long>& leaf_start, float*
 tb_status trsm_solve_2s(TrsmCtx& c, const std::vector<long>& leaf_start, float* B, long ldb, long rows, long cols);
 // One-time kernel attribute set-up for the grouped launches (not capturable).
 tb_status gemm_prepare_grouped();
-tb_status trsm_prepare_grouped();
 
 // General TRMM (side, uplo, trans, unit diagonal), tb_blas3.cu.
 // beta != 0 gives C = alpha op(A) B + beta C (the TRSM refinement residual).

@@ -589,8 +589,6 @@ tb_status recurse(TrsmCtx& c, long s, long e, const std::vector<long>& leaf_star
 
 }  // namespace
 
-tb_status trsm_prepare_grouped() { return TB_SUCCESS; }
-
 tb_status trsm_prep_launch(const PrepJobs& j, cudaStream_t st) {
   PrepDev p;
   memset(&p, 0, sizeof(p));
