@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(256) convert8_kernel(long long rows, long long
                                                        __half* __restrict__ lo, long long ldd, float lo_scale, int tri,
                                                        long long dup) {
   conv::convert8_body<WHOLE>(blockIdx.x, gridDim.x, blockIdx.y, gridDim.y, rows, cols, src, lds, al != 0, hi, lo, ldd,
-                      lo_scale, tri, dup);
+                             lo_scale, tri, dup);
 }
 
 // Scalar fallback for destinations that 16-byte stores cannot address.
@@ -90,7 +90,9 @@ tb_status convert_f32_f16(long long rows, long long cols, const float* src, long
   if (vec && conv::convert_whole(src, lds, rows))
     convert8_kernel<true><<<grid, threads, 0, stream>>>(rows, cols, src, lds, 1, hi, lo, ldd, lo_scale, tri, dup);
   else if (vec)
-    convert8_kernel<false><<<grid, threads, 0, stream>>>(rows, cols, src, lds, conv::convert_aligned(src, lds) ? 1 : 0, hi, lo, ldd, lo_scale, tri, dup);
+    convert8_kernel<false><<<grid, threads, 0, stream>>>(rows, cols, src, lds,
+                                                         conv::convert_aligned(src, lds) ? 1 : 0, hi, lo, ldd,
+                                                         lo_scale, tri, dup);
   else
     convert1_kernel<<<grid, threads, 0, stream>>>(rows, cols, src, lds, hi, lo, ldd, lo_scale, tri, dup);
   TB_CUDA_TRY(cudaGetLastError());

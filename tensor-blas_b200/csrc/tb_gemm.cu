@@ -117,9 +117,9 @@ bool make_c_map(CUtensorMap* map, float* C, long long rows, long long cols, long
 // previous grid on the stream still runs (once all of its CTAs have started),
 // do their set-up (barriers, TMEM allocation) and wait in grid_dep_wait until
 // that grid has completed. Chains of short launches gain most: on a B200 the
-// TRSM of 4096 x 256 (nb 256, 31 launches) took 483 us without it and 451
-// with, 4096 x 4096 (nb 512) 432 / 405, 8192 x 8192 1210 / 1151; order 16384 is
-// the same within the runs' spread. TB_PDL=0 in the environment (read once)
+// TRSM of 4096 x 256 (nb 256, 31 products) took 409 us without it and 339
+// with, 4096 x 4096 (nb 512) 417 / 367, 8192 x 8192 1196 / 1130; order 16384 is
+// the same within the runs' spread (5.74 / 5.76 ms). TB_PDL=0 in the environment (read once)
 // turns it off, with the same results. Launches into a stream under graph
 // capture are always plain.
 bool dependent_launch(cudaStream_t stream) {
@@ -194,9 +194,10 @@ tb_status launch_variant(const GemmArgs& args, int num_tiles, cudaStream_t strea
 
 // 4 K-blocks (256-deep) between folds: at n = k = 16384 on a B200 the split
 // SYRK / TRSM of an earlier tile shape took 12.51 / 16.43 ms with 2, 11.69 /
-// 15.18 ms with 4 and 11.22 / 14.01 ms with 8, at normwise errors vs FP64 of 2.8e-7 / 1.3e-7,
-// 3.7e-7 / 1.6e-7 and 6.6e-7 / 2.4e-7; 4 keeps the 1e-6 target with margin
-// as K grows.
+// 15.18 ms with 4 and 11.22 / 14.01 ms with 8, at normwise errors vs FP64 of
+// 2.8e-7 / 1.3e-7, 3.7e-7 / 1.6e-7 and 6.6e-7 / 2.4e-7; 4 keeps the 1e-6 target
+// with margin as K grows (U[-1, 1] operands: 4.0e-7 at K = 32768, 5.4e-7 at
+// 131072; operands of one sign, whose truncations add up: 1.1e-6 at any K).
 int split_kchunk() {
   static const int k = [] {
     const char* e = getenv("TB_SPLIT_KCHUNK");
@@ -316,7 +317,8 @@ tb_status gemm_launch(const GemmCall& c, cudaStream_t stream) {
   launch_variant<GemmCfg<BN, NS, AMN, BMN, PF>, false>(a, c.num_tiles, stream, c.flops, bytes)
   if (c.fp8) {
     if (c.pair) return TB_PAIR(false, false, PairMode::kFp8);
-    return launch_variant<GemmCfg<kGemmBNFp8, 1, false, false, false, true>, false>(a, c.num_tiles, stream, c.flops, bytes);
+    using Cfg = GemmCfg<kGemmBNFp8, 1, false, false, false, true>;
+    return launch_variant<Cfg, false>(a, c.num_tiles, stream, c.flops, bytes);
   }
   if (c.pair && split) TB_BY_LAYOUT(TB_PAIR, PairMode::kSplit);
   if (c.pair) {

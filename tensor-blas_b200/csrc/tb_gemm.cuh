@@ -107,8 +107,8 @@ __device__ __forceinline__ int static_next(const GemmArgs& a, int b, int nb, int
 
 // Tile hand-off inside a CTA under the device-side scheduler: the producer
 // claims a tile and queues its index (or -1, the end) in a kTileQ-deep ring;
-// the MMA issuer, the four epilogue warps and (prefetch variants) the C
-// loader each take the indices in order and release the slot.
+// the MMA issuer, the eight epilogue warps and the C loader each take the
+// indices in order and release the slot.
 constexpr int kTileQ = 4;
 
 // Split mode: main folds for which the correction stays in its accumulator (a
@@ -1072,15 +1072,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_cons
 // correction (one phase a stretch of kCorrRounds). Per 64-deep K block and SM the 256 x 256 tile
 // moves 64 KB into shared memory and 96 KB out of it for 1536 MMA cycles,
 // where 256 x 128 tiles (which left room to double-buffer) moved 96 + 144 KB.
-// The tensor pipe is 93 % busy while the SM is active against 65 %: SYR2K n = 16384, k = 4096 went from 6.0
-// to 5.3 ms.
+// The tensor pipe is 93 % busy while the SM is active against 65 %: SYR2K n =
+// 16384, k = 4096 went from 6.0 to 5.3 ms.
 // kFp8: e4m3 operands, one 128-deep K block a round (512 MMA cycles per SM),
 // the accumulators double-buffered and folded with the blocks' scales. The
-// path of a round's signals (commit, fold, release, next MMAs) bounds it: the
-// tensor pipe is 38 % busy, and with three quarters of the fold's work left
-// out an 8192 launch still takes 555 us of its 676. Single-CTA 128 x 128 tiles have 256 MMA cycles a round
-// and as long a path for a quarter of the work a pair does: SYMM 16384 went
-// from 8.8 to 6.6 ms.
+// path of a round's signals (commit, fold, release, next MMAs) bounds it: a
+// round takes about 1350 cycles, the tensor pipe is 38 % busy. Single-CTA 128 x
+// 128 tiles have 256 MMA cycles a round and nearly as long a path for a quarter
+// of the work a pair does: SYMM 16384 went from 8.8 to 6.6 ms.
 // The fold modes keep 128 sums per epilogue thread: the first four warps give
 // registers to the epilogue's eight (setmaxnreg: 128 x 72 + 256 x 216 = 384 x
 // 168, the launch's allocation).

@@ -117,14 +117,15 @@ struct GemmCall {
   long long ld_out = 0;
   float out_lo_scale = 2048.0f;
   int out_m = -1, out_n = -1;  // side-copy region (default: all of C)
-  int kblocks = 0;   // most K-blocks (64) of any tile; 0 < kblocks <= kGemmPfMaxKb selects the prefetch variants
+  int kblocks = 0;   // most K-blocks (64) of any tile; 0 < kblocks <= kGemmPfMaxKb: a short-K launch
   const int* ranges = nullptr;  // per-CTA tile ranges of a balanced list (set by gemm_launch_plan)
-  // FP8 (e4m3) operands: K-major byte matrices (Operand.ld in bytes), K
-  // blocks of 128, per-(128-row block, K block) scales (row-block-major,
-  // scale_ld K blocks per row block); tiles 128 x 128.
   bool pair = false;  // set by gemm_launch_plan: 256 x 256 tiles on CTA pairs (cta_group::2)
   int bn = 0;         // set by gemm_launch_plan: tile width of a single-CTA launch (0: gemm_bn(split, kblocks))
   int epi_cols = kEpiCols;  // columns of the TMA boxes C moves in (the persistent TRSM's kernel: 32)
+  // FP8 (e4m3) operands: K-major byte matrices (Operand.ld in bytes), K
+  // blocks of 128, per-(128-row block, K block) scales (row-block-major,
+  // scale_ld K blocks per row block; negative: the block is left out); plans of
+  // 128 x 128 tiles.
   bool fp8 = false;
   const float* scale_a = nullptr;
   const float* scale_b = nullptr;
@@ -134,8 +135,8 @@ struct GemmCall {
 };
 
 // Tile width along N used by the engine for a given split mode (and, with
-// kblocks = the most K-blocks of any tile, for the prefetch variants that
-// launches with short K ranges use: plain tiles are then 128 wide).
+// kblocks = the most K-blocks of any tile, for launches with short K ranges:
+// plain tiles are then 128 wide).
 constexpr int kGemmBM = 128;
 constexpr int kGemmBK = 64;
 constexpr int kGemmPfMaxKb = 16;

@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(kDiagThreads)
 template <class T>
 tb_status diag_inv32(long long n, const T* A, long long lda, double* D, bool unit, const WOut& out, cudaStream_t st) {
   constexpr int per = kDiagThreads / 32;
-  diag_inv32_kernel<T><<<(unsigned)(((n + 31) / 32 + per - 1) / per), kDiagThreads, per * sizeof(DiagSmem), st>>>(n, A, lda, D, unit,
-                                                                                           out);
+  const unsigned blocks = (unsigned)(((n + 31) / 32 + per - 1) / per);
+  diag_inv32_kernel<T><<<blocks, kDiagThreads, per * sizeof(DiagSmem), st>>>(n, A, lda, D, unit, out);
   TB_CUDA_TRY(cudaGetLastError());
   note_launch();
   return TB_SUCCESS;
@@ -602,7 +602,8 @@ tb_status trsm_prep_launch(const PrepJobs& j, cudaStream_t st) {
     const bool vec = conv::convert_vec(c.hi, c.lo, c.ldd, 0);
     long long gx = 0, gy = 0;
     conv::convert_grid(c.rows, c.cols, c.tri, vec, sm_count(), kPrepThreads, &gx, &gy);
-    p.conv_vec[k] = !vec ? 0 : conv::convert_whole(c.src, c.lds, c.rows) ? 3 : conv::convert_aligned(c.src, c.lds) ? 2 : 1;
+    const bool aligned = conv::convert_aligned(c.src, c.lds);
+    p.conv_vec[k] = !vec ? 0 : conv::convert_whole(c.src, c.lds, c.rows) ? 3 : aligned ? 2 : 1;
     p.conv_gx[k] = gx;
     p.conv_base[k] = next;
     p.conv_blocks[k] = gx * gy;

@@ -1059,8 +1059,9 @@ tb_status trsm_solve_dag(TrsmCtx& c, const std::vector<long>& leaf_start, float*
     TB_TRY(gemm_build_args(ops[i].call, &hops[i]));
     flops += ops[i].call.flops;
   }
-  // every output (B and the FP16 side copies) must leave through TMA stores,
-  // whose completion a tile waits for before it publishes its progress
+  // B must leave through TMA stores, whose completion a tile waits for before
+  // it publishes its progress (the FP16 side copies are plain stores, fenced
+  // before that)
   for (size_t i = 0; i < ops.size(); ++i)
     if (!hops[i].tma_c)
       return trsm_solve_launches(c, leaf_start, B, ldb, rows, cols);
